@@ -35,40 +35,24 @@ N_ENVS = 16384
 WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs per GPU, "
             "FK (all link poses) + WORLD Jacobian + CRBA + RNEA + ABA per env per step")
 
-# FP64 thread-instructions (DFMA + DMUL + DADD) per environment-step and DRAM bytes per
-# environment of one step (structure-of-arrays buffers; both launches when the step is split),
-# from an ncu capture of the model-specialised kernels (run-time compiled) and of the generic
-# ones. They hold for the
-# kernel source whose digest is KERNEL_SOURCE_SHA256 (kernel_source_digest()); a CPU test
-# fails when the source changes, so the figures are re-captured with every kernel change.
-KERNEL_COUNTERS = {
-    # two launches (FK + Jacobian: 507,392 FP64 warp instructions; CRBA + RNEA + ABA with
-    # forward dynamics from the mass matrix: 1,650,688) per 16384 environments (the thread
-    # counts with all predicates on, 987.6 + 3223.0 per environment, agree); DRAM bytes as
-    # ncu counted them in a cold capture, where most of the 29 MB of results is still held in
-    # L2 when the launches end
-    "specialised": {"fp64_inst_per_env": 2158080 * 32 / 16384, "dram_bytes_per_env": 8.32e6 / 16384},
-}
-KERNEL_SOURCE_SHA256 = "49e104c5e570e5883a86511be471883515b1e9846a8d8e5c713b105010c2b432"
-KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "step_kernel.cuh")
-STEP_OPS = (3, 28)  # sgdyn_step at N = 16384: FK + Jacobian beside CRBA + RNEA + ABA, two launches
+# FP64 thread-instructions (DFMA + DMUL + DADD), warp instructions and DRAM bytes per
+# environment of one five-op step (structure-of-arrays buffers), from an ncu capture of the
+# block sweep at 16384 environments. They hold for the kernel source whose digest is
+# KERNEL_SOURCE_SHA256 (kernel_source_digest()); a CPU test fails when the source changes, so
+# the figures are re-captured with every kernel change. DRAM bytes as ncu counted them in a cold
+# capture: the inputs are read, the 29 MB of results are still held in L2 when the launch ends.
+KERNEL = "block floating point"
+KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 38812134 / 16384,
+                   "dram_bytes_per_env": 4.87e6 / 16384}
+KERNEL_SOURCE_SHA256 = "21c7ace5e600a79555459697eb41c3721558f6dfbf8f408a44ae6b46ceb19556"
+KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 
-def kernel_source_digest(model, ops=None):
-    """SHA-256 of what the step kernels of `model` are compiled from: the run-time-generated
-    translation units (their floating-point constants masked: the last bits of the model
-    tables differ between host libms, the instruction stream does not) and the device headers
-    they include. `ops` defaults to the two launches of the five-op step as bench.py runs it."""
+def kernel_source_digest(model=None):
+    """SHA-256 of the headers that the step kernel is compiled from (one kernel for all models)."""
     import hashlib
-    import re
-
-    from sapien_gb300 import _native as N
 
     h = hashlib.sha256()
-    for o in (STEP_OPS if ops is None else (ops,)):
-        src = ctypes.c_char_p()
-        N.check(N.load().sgdyn_jit_source(model._h, o, ctypes.byref(src)))
-        h.update(re.sub(rb"[-+]?(?:(?:\d+\.\d*|\.\d+)(?:[eE][-+]?\d+)?|\d+[eE][-+]?\d+)", b"#", src.value))
     for name in KERNEL_HEADERS:
         with open(os.path.join(ROOT, "sapien_gb300", "csrc", name), "rb") as f:
             h.update(f.read())
@@ -674,8 +658,6 @@ def main():
     poses, J, M, tau_o, qdd_o = (torch.empty(c, n, dtype=torch.float64, device=dev) for c in out_cols)
     pm._prepare(dev)
     L = N.load()
-    kernel = "specialised" if L.sgdyn_jit_prepare(pm._h, N.OP_ALL) == 0 else "generic"
-    counters = KERNEL_COUNTERS.get(kernel)  # None for the generic kernels (not captured)
     stream = torch.cuda.current_stream(dev)
     sp = ctypes.c_void_p(stream.cuda_stream)
     P = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
@@ -689,14 +671,7 @@ def main():
             raise RuntimeError(N.last_error())
 
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)  # > 129 MB L2
-    # sgdyn_step runs the five ops as two concurrent launches (FK + Jacobian beside CRBA +
-    # RNEA + ABA) while one warp per 32 environments gives fewer than two warps per FP64
-    # scheduler (split mode 2, the default)
-    mode = ctypes.c_int()
-    N.check(L.sgdyn_step_split(-1, ctypes.byref(mode)))
-    sms = torch.cuda.get_device_properties(dev).multi_processor_count
-    split = mode.value == 1 or (mode.value == 2 and (n + 31) // 32 < 2 * 4 * sms)
-    launches_per_step = 2 if split else 1
+    launches_per_step = 1  # the five ops in one launch (automatic settings)
 
     # ---- kernel-only timing, inputs resident in HBM ---------------------------------
     for _ in range(args.warmup):
@@ -818,7 +793,7 @@ def main():
     achieved_gbs = alg / (ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved_gbs, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved_gbs / peaks["hbm_gbs"],
-                "traffic": counters["dram_bytes_per_env"] * n if counters else None,
+                "traffic": KERNEL_COUNTERS["dram_bytes_per_env"] * n,
                 "peak_source": f"{peak_src} (MEASURED_PEAKS.json hbm_gbs)",
                 "algorithmic_bytes_per_launch": alg}
     dfma = fp64_peak_dfma_per_s()
@@ -827,16 +802,16 @@ def main():
     if dfma:
         peak_gflops = 2 * dfma / 1e9  # one DFMA = 2 flops
         ach = alg["step"] * n / (ms * 1e-3) / 1e9
-        issued = counters["fp64_inst_per_env"] * n / (ms * 1e-3) / 1e9 if counters else None
+        issued = KERNEL_COUNTERS["fp64_inst_per_env"] * n / (ms * 1e-3) / 1e9
         roofline_fp64 = {
             "bound": "fp64", "unit": "GFLOP/s", "peak": peak_gflops,
             "peak_source": "measured live: DFMA chain microbenchmark (bench_fp64_peak.cu), 2 flops per DFMA",
             "algorithmic_flops_per_env": alg["step"], "achieved": ach, "frac": ach / peak_gflops,
             "algorithmic_source": "oracle counting scalar: local-frame recursions, operations on structural "
                                   "zeros and ones skipped; the kernels' world-frame sweep needs fewer",
-            "issued_inst_per_env": counters["fp64_inst_per_env"] if counters else None,
-            "issued_inst_per_s": issued * 1e9 if counters else None,
-            "issued_frac": issued / (dfma / 1e9) if counters else None,
+            "issued_inst_per_env": KERNEL_COUNTERS["fp64_inst_per_env"],
+            "issued_inst_per_s": issued * 1e9,
+            "issued_frac": issued / (dfma / 1e9),
             "issued_source": "ncu sass FP64 instruction counts of this kernel source "
                              f"(sha256 {KERNEL_SOURCE_SHA256[:12] or 'unset'}); frac against the DFMA issue peak",
             "source_matches_counters": kernel_source_digest(pm) == KERNEL_SOURCE_SHA256,
@@ -888,10 +863,9 @@ def main():
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True, "scaling": "weak",
         "vs_baseline": None, "dtype": "f64", "data": "synthetic",
         "config": workload_config(n, nv, nl),
-        "execution": {"parallelism": f"data-parallel replicas over environments x{world}", "kernel": kernel,
+        "execution": {"parallelism": f"data-parallel replicas over environments x{world}", "kernel": KERNEL,
                       "launches_per_step": launches_per_step,
-                      "step": "FK+Jacobian and CRBA+RNEA+ABA as two concurrent launches" if split
-                      else "one fused launch"},
+                      "step": "one fused launch"},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
                 "ms_per_step": ms_e2e,
                 "transfer": "sgdyn_step on mapped pinned host buffers (SoA): the kernel reads inputs from and "

@@ -182,6 +182,8 @@ int choose_lanes(Model& M, int64_t n) {
   return best;
 }
 
+BfpTree bfp_tree(const Model& M) { return {M.njoints(), M.nv(), M.nq_ext(), M.btree().npairs, M.btree().nints}; }
+
 int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const double* qd, const double* qdd,
              const double* tau, double* poses, double* J, double* M, double* tau_out, double* qdd_out, int layout,
              void* stream) {
@@ -220,6 +222,18 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
   a.tau_out = make_arr(tau_out, n, nv, layout);
   a.qdd_out = make_arr(qdd_out, n, nv, layout);
   auto s = static_cast<cudaStream_t>(stream);
+  // With every setting automatic: the block-floating-point sweep, one launch for any op set and
+  // batch size (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings
+  // (lanes, split, forward-dynamics route) and what that sweep cannot hold.
+  int fd_mode = 0;
+  fd_method(-1, &fd_mode);
+  if (Mo.bfp_ok() && Mo.lanes == 0 && g_split_mode.load() == 2 && fd_mode == 0 &&
+      !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
+    const cudaError_t e = launch_bfp_step(dm, bfp_tree(Mo), ops, a, s);
+    if (e == cudaSuccess) return SGDYN_OK;
+    if (e != cudaErrorNotSupported)
+      return fail(SGDYN_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString(e));
+  }
   static const int fused[] = {OP_ALL, OP_CRBA | OP_RNEA | OP_ABA, OP_RNEA | OP_ABA, OP_FK | OP_JAC};
   int rest = ops;
   std::vector<int> launches;

@@ -27,6 +27,42 @@ typedef unsigned long size_t;
 
 namespace sgdyn {
 
+// Constants of a joint and of a link as block-floating-point mantissas (bfp.cuh): rotations and
+// the axis of exponent -60, the others with the exponents pe, me, ce, Ie. The body inertia is
+// kept as mass, centre of mass and rotational inertia about it.
+struct alignas(16) BJoint {
+  long long R[9], p[3], axis[3], m, c[3], I[6];
+  int pe, me, ce, Ie;
+  long long pad_;
+};
+static_assert(sizeof(BJoint) == 224, "BJoint layout");
+struct alignas(16) BLink {
+  long long R[9], p[3];
+  int pe, pad_[3];
+};
+static_assert(sizeof(BLink) == 112, "BLink layout");
+
+// The tree as the block sweeps (bfp_block.cuh) walk it: `off` entries index the int array that
+// follows. Tree columns are velocity indices in depth-first order; a column's depth counts the
+// columns above it; a pair is a column with itself or one of its ancestor columns, pairs of a
+// column in order of depth, so that pair (a, c) is number row_start[a] + depth(c).
+struct alignas(16) BTree {
+  int levels;      // joint levels
+  int npairs;
+  int col_levels;  // column depths
+  int nints;       // without pair_of
+  int parent, end, level;  // [nj] each: DJoint::parent, subtree_end, level from 1
+  int order;       // [nj - 1] joints by level
+  int level_start; // [levels + 1]
+  int col_joint, col_dof, col_depth, col_ext, row_start;  // [nv] each
+  int col_order;   // [nv] columns by depth
+  int col_level_start;  // [col_levels + 1]
+  int pair_row, pair_col;  // [npairs] each
+  int pair_of;     // [nv * nv], after the others: pair of an external row and column, -1 where M is 0
+  int pad_;
+};
+static_assert(sizeof(BTree) == 80, "BTree layout");
+
 enum JointKind : int { JK_NONE = 0, JK_REVOLUTE = 1, JK_PRISMATIC = 2, JK_CONTINUOUS = 3, JK_FREEFLYER = 4 };
 enum AxisKind : int { AX_X = 0, AX_Y = 1, AX_Z = 2, AX_GENERAL = 3 };
 enum JointFlags : int { JF_ROT_IDENTITY = 1 };
@@ -94,6 +130,17 @@ SG_HD const DFrame* model_frames(const DModel* m) {
 SG_HD size_t model_table_bytes(int nj, int nlinks) {
   return sizeof(DModel) + sizeof(DJoint) * size_t(nj) + sizeof(DLink) * size_t(nlinks) +
          sizeof(DFrame) * size_t(nj);
+}
+// The block-floating-point constants follow the frames in a model's device copy.
+SG_HD const BJoint* model_bjoints(const DModel* m) {
+  return reinterpret_cast<const BJoint*>(reinterpret_cast<const char*>(m) + model_table_bytes(m->nj, m->nlinks));
+}
+SG_HD const BLink* model_blinks(const DModel* m) { return reinterpret_cast<const BLink*>(model_bjoints(m) + m->nj); }
+SG_HD const BTree* model_btree(const DModel* m) {
+  return reinterpret_cast<const BTree*>(model_blinks(m) + m->nlinks);
+}
+SG_HD size_t model_bfp_bytes(int nj, int nlinks) {
+  return sizeof(BJoint) * size_t(nj) + sizeof(BLink) * size_t(nlinks);
 }
 
 }  // namespace sgdyn

@@ -108,6 +108,13 @@ int stash_bucket(int nj);
 
 // Fused world-frame sweep: any subset of {FK poses, full WORLD Jacobian, CRBA, RNEA, ABA}.
 cudaError_t launch_step(const DModel* dm, int nj, int ops, const StepArgs& a, cudaStream_t s);
+// The same sweep in block floating point with a block of threads per group of environments
+// (bfp_block.cuh); BfpTree: the model's sizes (tree_ints: BTree::nints). cudaErrorNotSupported (nothing launched) when an
+// environment's state is too large for it.
+struct BfpTree {
+  int nj, nv, nq, npairs, tree_ints;
+};
+cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s);
 // Forward dynamics alone with three lanes per environment (team3.cuh; one-DoF joints and a
 // free-flyer root).
 cudaError_t launch_aba3(const DModel* dm, int nj, const StepArgs& a, cudaStream_t s);

@@ -592,6 +592,7 @@ void Model::rebuild_table() {
     dl[l].joint = B.joint;
     dl[l].flags = is_identity(dl[l].R) ? JF_ROT_IDENTITY : 0;
   }
+  rebuild_bfp();
   // device copies are stale now
   for (auto& kv : dev_) {
     int cur;
@@ -614,6 +615,160 @@ void Model::rebuild_table() {
   team_cp_.clear();
 }
 
+namespace {
+// x 2^-e rounded to a mantissa
+long long mantissa(long double x, int e) { return std::llrint(std::ldexp(x, -e)); }
+// The exponent that puts the largest magnitude of v[0..n) in [2^60, 2^61).
+int block_exponent(const long double* v, int n) {
+  long double m = 0;
+  for (int k = 0; k < n; k++) m = std::max(m, std::fabs(v[k]));
+  if (m == 0) return -1000;
+  int e;
+  std::frexp(m, &e);  // m = f 2^e, 1/2 <= f < 1
+  return e - 61;
+}
+int to_block(const long double* v, int n, long long* out) {
+  int e = block_exponent(v, n);
+  for (int k = 0; k < n; k++)
+    if (std::llabs(mantissa(v[k], e)) >= (1LL << 61)) e++;  // rounded up to the next power of two
+  for (int k = 0; k < n; k++) out[k] = mantissa(v[k], e);
+  return e;
+}
+bool in_range(const double* v, int n) {
+  for (int k = 0; k < n; k++)
+    if (!(v[k] == 0 || (std::fabs(v[k]) > 0x1p-100 && std::fabs(v[k]) < 0x1p100))) return false;
+  return true;
+}
+}  // namespace
+
+// BJoint / BLink from the FP64 tables; the centre of mass and the inertia about it in extended
+// precision, so that the constants lose nothing against their FP64 form.
+void Model::rebuild_bfp() {
+  const auto* hdr = reinterpret_cast<const DModel*>(table_.data());
+  const DJoint* J = model_joints(hdr);
+  const DLink* L = model_links(hdr);
+  bfp_.assign(model_bfp_bytes(hdr->nj, hdr->nlinks), 0);
+  auto* bj = reinterpret_cast<BJoint*>(bfp_.data());
+  auto* bl = reinterpret_cast<BLink*>(bj + hdr->nj);
+  bfp_ok_ = in_range(hdr->gravity, 3);
+  for (int i = 1; i < hdr->nj; i++) {
+    const DJoint& d = J[i];
+    BJoint& b = bj[i];
+    bfp_ok_ = bfp_ok_ && in_range(d.R, 9) && in_range(d.p, 3) && in_range(d.axis, 3) && in_range(&d.m, 1) &&
+              in_range(d.h, 3) && in_range(d.I, 6) && d.m >= 0;
+    if (d.m == 0) bfp_ok_ = bfp_ok_ && d.h[0] == 0 && d.h[1] == 0 && d.h[2] == 0;
+  }
+  for (int l = 0; l < hdr->nlinks; l++) bfp_ok_ = bfp_ok_ && in_range(L[l].R, 9) && in_range(L[l].p, 3);
+  // rotations and axes of exponent -60 need entries of at most 1
+  auto unit = [&](const double* v, int n) {
+    for (int k = 0; k < n; k++) bfp_ok_ = bfp_ok_ && std::fabs(v[k]) < 1 + 1e-6;
+  };
+  for (int i = 1; i < hdr->nj; i++) {
+    unit(J[i].R, 9);
+    unit(J[i].axis, 3);
+  }
+  for (int l = 0; l < hdr->nlinks; l++) unit(L[l].R, 9);
+  // every joint's parent before it, in the joint and the column numbering
+  for (int i = 1; i < hdr->nj; i++)
+    if (J[i].parent >= i || (J[i].parent > 0 && J[J[i].parent].ivx + J[J[i].parent].nv > J[i].ivx)) bfp_ok_ = false;
+  if (!bfp_ok_) return;
+  for (int i = 1; i < hdr->nj; i++) {
+    const DJoint& d = J[i];
+    BJoint& b = bj[i];
+    for (int k = 0; k < 9; k++) b.R[k] = mantissa(d.R[k], -60);
+    for (int k = 0; k < 3; k++) b.axis[k] = mantissa(d.axis[k], -60);
+    const long double p[3] = {d.p[0], d.p[1], d.p[2]};
+    b.pe = to_block(p, 3, b.p);
+    const long double m = d.m;
+    b.me = to_block(&m, 1, &b.m);
+    long double c[3] = {0, 0, 0};
+    if (d.m > 0)
+      for (int k = 0; k < 3; k++) c[k] = d.h[k] / m;
+    b.ce = to_block(c, 3, b.c);
+    const long double cc = c[0] * c[0] + c[1] * c[1] + c[2] * c[2];
+    const long double I[6] = {d.I[0] - m * (cc - c[0] * c[0]), d.I[1] + m * c[0] * c[1], d.I[2] + m * c[0] * c[2],
+                              d.I[3] - m * (cc - c[1] * c[1]), d.I[4] + m * c[1] * c[2],
+                              d.I[5] - m * (cc - c[2] * c[2])};
+    b.Ie = to_block(I, 6, b.I);
+  }
+  for (int l = 0; l < hdr->nlinks; l++) {
+    for (int k = 0; k < 9; k++) bl[l].R[k] = mantissa(L[l].R[k], -60);
+    const long double p[3] = {L[l].p[0], L[l].p[1], L[l].p[2]};
+    bl[l].pe = to_block(p, 3, bl[l].p);
+  }
+  // levels, columns and pairs
+  const int nj = hdr->nj, nv = hdr->nv;
+  std::vector<int> ints, level(nj, 0), par(nv, -1), dep(nv, 0), cj(nv), ck(nv), ext(nv), rs(nv), pr, pc;
+  BTree t{};
+  for (int i = 1; i < nj; i++) {
+    const int p = J[i].parent;
+    level[i] = p > 0 ? level[p] + 1 : 1;
+    t.levels = std::max(t.levels, level[i]);
+    for (int k = 0; k < J[i].nv; k++) {
+      const int a = J[i].ivx + k;
+      par[a] = k > 0 ? a - 1 : (p > 0 ? J[p].ivx + J[p].nv - 1 : -1);
+      dep[a] = par[a] >= 0 ? dep[par[a]] + 1 : 0;
+      t.col_levels = std::max(t.col_levels, dep[a] + 1);
+      cj[a] = i;
+      ck[a] = k;
+      ext[a] = J[i].vcol + k;
+    }
+  }
+  for (int a = 0; a < nv; a++) {
+    rs[a] = int(pr.size());
+    std::vector<int> up;
+    for (int c = a; c >= 0; c = par[c]) up.push_back(c);
+    for (size_t k = up.size(); k-- > 0;) {
+      pr.push_back(a);
+      pc.push_back(up[k]);
+    }
+  }
+  t.npairs = int(pr.size());
+  auto put = [&](const std::vector<int>& v) {
+    const int at = int(ints.size());
+    ints.insert(ints.end(), v.begin(), v.end());
+    return at;
+  };
+  auto by_level = [&](int lo, int hi, int first, int n, const std::vector<int>& lv, int* order, int* start) {
+    std::vector<int> o, s;
+    for (int d = first; d < first + n; d++) {
+      s.push_back(int(o.size()));
+      for (int i = lo; i < hi; i++)
+        if (lv[i] == d) o.push_back(i);
+    }
+    s.push_back(int(o.size()));
+    *order = put(o);
+    *start = put(s);
+  };
+  std::vector<int> parent(nj, 0), end(nj, 0);
+  for (int i = 1; i < nj; i++) {
+    parent[i] = J[i].parent;
+    end[i] = J[i].subtree_end;
+  }
+  t.parent = put(parent);
+  t.end = put(end);
+  t.level = put(level);
+  by_level(1, nj, 1, t.levels, level, &t.order, &t.level_start);
+  t.col_joint = put(cj);
+  t.col_dof = put(ck);
+  t.col_depth = put(dep);
+  t.col_ext = put(ext);
+  t.row_start = put(rs);
+  by_level(0, nv, 0, t.col_levels, dep, &t.col_order, &t.col_level_start);
+  t.pair_row = put(pr);
+  t.pair_col = put(pc);
+  std::vector<int> of(size_t(nv) * nv, -1);
+  for (int i = 0; i < t.npairs; i++) of[ext[pr[i]] * nv + ext[pc[i]]] = of[ext[pc[i]] * nv + ext[pr[i]]] = i;
+  t.nints = int(ints.size());
+  t.pair_of = put(of);
+  while (ints.size() % 4) ints.push_back(0);
+  btree_ = t;
+  const size_t at = bfp_.size();
+  bfp_.resize(at + sizeof(BTree) + 4 * ints.size());
+  std::memcpy(bfp_.data() + at, &t, sizeof(BTree));
+  std::memcpy(bfp_.data() + at + sizeof(BTree), ints.data(), 4 * ints.size());
+}
+
 const DModel* Model::device_table(int* err) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
@@ -624,11 +779,13 @@ const DModel* Model::device_table(int* err) {
   auto it = dev_.find(dev);
   if (it != dev_.end()) return static_cast<const DModel*>(it->second);
   void* p = nullptr;
-  if (cudaMalloc(&p, table_.size()) != cudaSuccess) {
+  if (cudaMalloc(&p, table_.size() + bfp_.size()) != cudaSuccess) {
     *err = 2;
     return nullptr;
   }
-  if (cudaMemcpy(p, table_.data(), table_.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+  if (cudaMemcpy(p, table_.data(), table_.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+      (!bfp_.empty() && cudaMemcpy(static_cast<unsigned char*>(p) + table_.size(), bfp_.data(), bfp_.size(),
+                                   cudaMemcpyHostToDevice) != cudaSuccess)) {
     cudaFree(p);
     *err = 3;
     return nullptr;

@@ -103,6 +103,12 @@ class Model {
   const DModel* find_device_table();
   // Host copy of the packed table (for tests and for the heterogeneous packer).
   const std::vector<unsigned char>& host_table() const { return table_; }
+  // The block-floating-point constants (BJoint per joint, then BLink per link), and whether
+  // every constant of the model is zero or within 2^+-100, as those sweeps need. After them the
+  // BTree and its ints.
+  const std::vector<unsigned char>& bfp_table() const { return bfp_; }
+  bool bfp_ok() const { return bfp_ok_; }
+  const BTree& btree() const { return btree_; }
 
   // Team table for L lanes per environment (layout in step_kernel.cuh: TeamLanes);
   // *critical_path receives the joint-cost length of the trunk + heaviest lane.
@@ -130,10 +136,14 @@ class Model {
 
  private:
   void rebuild_table();
+  void rebuild_bfp();
   int nq_ext_ = 0, nv_ = 0, nq_int_ = 0;
   std::vector<int> qcol_, vcol_;   // per joint: external q / v column of its first coordinate
   std::vector<int> link_bodies_;   // external link index -> bodies[]
   std::vector<unsigned char> table_;
+  std::vector<unsigned char> bfp_;
+  bool bfp_ok_ = false;
+  BTree btree_{};
   std::map<int, void*> dev_;       // device ordinal -> device copy of table_
   std::map<std::pair<int, int>, void*> dev_team_;  // (device, L) -> device team table
   std::map<int, int> team_cp_;                       // L -> critical path

@@ -1,0 +1,135 @@
+"""The block-floating-point sweeps (csrc/bfp_block.cuh), which every batched
+call takes with its settings automatic, against the oracle and against the FP64 sweeps that
+forced settings select. Sizes around the edges of their blocks (4 to 32 environments, fewer per
+block while there are few blocks), both layouts, and inputs that send single environments of a
+block to the FP64 algebra."""
+import contextlib
+import ctypes
+
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from sapien_gb300 import PinocchioModel, synthetic as syn
+from sapien_gb300 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+ROBOTS = {
+    "slide": lambda: syn.serial_chain(1, seed=2, kinds=["prismatic"]),
+    "mixed": lambda: syn.serial_chain(6, seed=11, kinds=["revolute", "continuous", "prismatic", "revolute",
+                                                         "continuous", "prismatic"]),
+    "arm9": lambda: syn.arm_with_fingers(sapien_style=True),
+    "quadruped": syn.quadruped,
+    "humanoid": lambda: syn.humanoid(sapien_style=True),
+    "chain40": lambda: syn.serial_chain(40, seed=23),
+}
+
+
+def pair(robot):
+    pm, o = PinocchioModel(robot.urdf, [0, 0, -9.81]), Oracle(robot.urdf)
+    for m in (pm, o):
+        m.set_joint_order(robot.joint_names)
+        m.set_link_order(robot.link_names)
+    return pm, o
+
+
+def rel_per_env(g, o):
+    g, o = g.reshape(g.shape[0], -1), o.reshape(o.shape[0], -1)
+    return (np.abs(g - o).max(axis=1) / np.maximum(np.abs(o).max(axis=1), 1e-300)).max()
+
+
+@contextlib.contextmanager
+def fp64_route():
+    """One fused FP64 launch for every batched sweep; one lane for rollouts."""
+    L = N.load()
+    try:
+        assert L.sgdyn_step_split(0, None) == N.OK and L.sgdyn_rollout_lanes(1, None) == N.OK
+        yield
+    finally:
+        L.sgdyn_step_split(2, None)
+        L.sgdyn_rollout_lanes(0, None)
+
+
+def cuda(*arrays):
+    import torch
+
+    return [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in arrays]
+
+
+def host(out):
+    return {k: v.cpu().numpy() for k, v in out.items()}
+
+
+@pytest.mark.parametrize("name,n", [("slide", 1), ("slide", 33), ("mixed", 7), ("mixed", 2433), ("arm9", 4865),
+                                    ("arm9", 9729), ("quadruped", 31), ("quadruped", 4900), ("humanoid", 9),
+                                    ("chain40", 5)])
+def test_sweep_at_block_edges(name, n):
+    """The last environments of a batch that fills its last block partly (block sizes change at
+    8, 16 and 32 environments times two blocks per multiprocessor), every op set's outputs
+    against the oracle."""
+    robot = ROBOTS[name]()
+    pm, o = pair(robot)
+    ins = robot.sample(n, seed=n)
+    tail = slice(max(0, n - 40), n)
+    r = o.batch_step(*(a[tail] for a in ins), nthreads=8)
+    dev = cuda(*ins)
+    p = r["poses"][..., :12].reshape(tail.stop - tail.start, -1, 12)[..., 9:12]
+    for ops in (N.OP_ALL, N.OP_MASS_MATRIX, N.OP_INVERSE_DYNAMICS, N.OP_FORWARD_DYNAMICS, N.OP_JACOBIAN, N.OP_FK):
+        g = {k: v[tail] for k, v in host(pm.step_batched(*dev, ops=ops)).items()}
+        for k, w, tol in (("jacobian", r["J"], 1e-12), ("mass_matrix", r["M"], 1e-12), ("qf", r["tau"], 1e-12),
+                          ("qacc", r["qdd"], 1e-8)):
+            if k in g:
+                assert rel_per_env(g[k], w) <= tol, (ops, k)
+        if "link_poses" in g:
+            assert np.abs(g["link_poses"][..., :3] - p).max() <= 1e-12 * max(1.0, np.abs(p).max())
+
+
+@pytest.mark.parametrize("name", ["mixed", "arm9", "quadruped"])
+def test_refused_environments_match_fp64(name):
+    """Environments out of the range of block floating point (beyond 2^+-200, not finite, a
+    quaternion off unit length) come from the FP64 algebra of the same kernel; their neighbours
+    in the block are those of the clean batch, bit for bit."""
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    n = 70
+    q, qd, qdd, tau = robot.sample(n, seed=3)
+    clean = host(pm.step_batched(*cuda(q, qd, qdd, tau)))
+    qd[5] *= 1e70
+    qdd[17, 0] = 1e-90
+    tau[33] *= 1e75
+    q[40, -1] = 1e-80
+    odd = [5, 17, 33, 40]
+    if robot.nq_ext > robot.nv:
+        q[60, 3:7] *= 1.2
+        odd.append(60)
+    bad = [12, 50]
+    qd[12, 0] = np.nan
+    q[50, 0] = np.inf
+    g = host(pm.step_batched(*cuda(q, qd, qdd, tau)))
+    with fp64_route():
+        w = host(pm.step_batched(*cuda(q, qd, qdd, tau)))
+    rest = [e for e in range(n) if e not in odd + bad]
+    for k in clean:
+        assert np.array_equal(g[k][rest], clean[k][rest]), k
+        assert rel_per_env(g[k][odd], w[k][odd]) <= 1e-9, k
+        for e in bad:
+            assert np.isfinite(g[k][e]).all() == np.isfinite(w[k][e]).all(), (k, e)
+
+
+@pytest.mark.parametrize("name,n", [("mixed", 45), ("arm9", 2500), ("quadruped", 11), ("humanoid", 6)])
+def test_structure_of_arrays_equals_env_major(name, n):
+    import torch
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    ins = cuda(*robot.sample(n, seed=4))
+    want = pm.step_batched(*ins)
+    soa = [t.t().contiguous() for t in ins]
+    keys = ("link_poses", "jacobian", "mass_matrix", "qf", "qacc")
+    outs = [torch.full((want[k].numel() // n, n), float("nan"), dtype=torch.float64, device="cuda") for k in keys]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    N.check(N.load().sgdyn_step(pm._h, n, N.OP_ALL, *[p(t) for t in soa + outs], N.COL_MAJOR,
+                                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    for k, o in zip(keys, outs):
+        assert torch.equal(o.t().reshape(want[k].shape), want[k]), k
