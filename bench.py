@@ -42,9 +42,9 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 # the figures are re-captured with every kernel change. DRAM bytes as ncu counted them in a cold
 # capture: the inputs are read, the 29 MB of results are still held in L2 when the launch ends.
 KERNEL = "block floating point"
-KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 38812134 / 16384,
+KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39012326 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "21c7ace5e600a79555459697eb41c3721558f6dfbf8f408a44ae6b46ceb19556"
+KERNEL_SOURCE_SHA256 = "b68f3c723a19196d60fa94897df9c9cb8f7b289f787c74717f921a1adf9db3ae"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

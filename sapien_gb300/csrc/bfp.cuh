@@ -106,7 +106,9 @@ SG_HD i64 prod(Half a, Half b, Half c, Half d, Half f, Half g) {
   return wide(f.h, g.h,
               wide(c.h, d.h, wide(a.h, b.h, cross_terms(f, g, cross_terms(c, d, cross_terms(a, b, kRound))) >> 32)));
 }
-SG_HD Half neg(Half a) { return Half{-a.h, -a.l}; }
+// (the low half -2^31, of which there is no opposite, becomes 2^31 - 1: one unit of the mantissa)
+SG_HD int neg_low(int l) { return -imax(l, -2147483647); }
+SG_HD Half neg(Half a) { return Half{-a.h, neg_low(a.l)}; }
 
 // Operands of at most 2^60 with the high half also held times 4, for products in units of 2^60:
 // numbers of exponent -60 stay in that exponent.
@@ -117,7 +119,7 @@ SG_HD Half4 split4(i64 m) {
   const Half a = split(m);
   return Half4{a.h, a.l, int(unsigned(a.h) << 2)};
 }
-SG_HD Half4 neg(Half4 a) { return Half4{-a.h, -a.l, -a.h4}; }
+SG_HD Half4 neg(Half4 a) { return Half4{-a.h, neg_low(a.l), -a.h4}; }
 SG_HD i64 cross_terms(Half4 a, Half4 b, i64 c) { return wide(a.l, b.h, wide(a.h, b.l, c)); }
 constexpr i64 kRound4 = 1LL << 27;
 SG_HD i64 mul60(Half4 a, Half4 b) { return wide(a.h4, b.h4, cross_terms(a, b, kRound4) >> 28); }

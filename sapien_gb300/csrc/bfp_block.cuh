@@ -18,10 +18,10 @@
 //
 // Measured (GB300, device time per call; before: the FP64 sweeps, specialised per model or in
 // teams of lanes, that still serve forced settings and models out of range). All five ops: 7-DoF
-// arm, 16 environments 143 -> 32 us, 1000: 145 -> 36 us; 9-DoF arm, 16384: 156 -> 95 us. CRBA +
-// RNEA + forward dynamics: 9-DoF arm, 131071: 791 -> 541 us; 35-DoF humanoid, 1024: 422 -> 78 us.
+// arm, 16 environments 143 -> 32 us, 1000: 145 -> 36 us; 9-DoF arm, 16384: 156 -> 96 us. CRBA +
+// RNEA + forward dynamics: 9-DoF arm, 131071: 792 -> 544 us; 35-DoF humanoid, 1024: 422 -> 78 us.
 // Forward dynamics alone, 18-DoF quadruped, 3001: 84 -> 43 us. What bounds it at 16384 9-DoF
-// arms: 2369 warp instructions per environment (170 of its thread instructions in FP64, before
+// arms: 2381 warp instructions per environment (170 of its thread instructions in FP64, before
 // 4215) issued at 34 % of the schedulers' rate, waiting at barriers and for instruction fetch.
 #pragma once
 #include "bfp.cuh"

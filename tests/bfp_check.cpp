@@ -46,6 +46,21 @@ int main() {
     if (bfp::to_double(bfp::from_double(y)) != y || bfp::to_double(bfp::from_double(-y)) != -y) return 1;
   }
   std::printf("sin %.3Lg\ncos %.3Lg\nreciprocal %.3Lg\nrsqrt %.3Lg\nrounding %.3Lg\n", s, c, r, q, out);
+  // mantissas whose halves are the extreme ones: largest error of a cross product, relative to the norms
+  L edge = 0;
+  const unsigned lows[6] = {0x80000000u, 0x7fffffffu, 0xffffffffu, 0u, 1u, 0x80000001u};
+  auto mantissa = [&] { return (long long)((((unsigned long long)(U(-0x1p28, 0x1p28))) << 32) | lows[g() % 6]); };
+  for (int i = 0; i < 100000; i++) {
+    const bfp::Vec a{mantissa(), mantissa(), mantissa(), 0}, b{mantissa(), mantissa(), mantissa(), 0};
+    const bfp::Vec k = bfp::cross(a, b);
+    const L A[3] = {L(a.x), L(a.y), L(a.z)}, B[3] = {L(b.x), L(b.y), L(b.z)};
+    const L w[3] = {A[1] * B[2] - A[2] * B[1], A[2] * B[0] - A[0] * B[2], A[0] * B[1] - A[1] * B[0]};
+    const L x[3] = {val(k.x, k.e), val(k.y, k.e), val(k.z, k.e)};
+    for (int j = 0; j < 3; j++) edge = fmaxl(edge, fabsl(x[j] - w[j]) * 0x1p-120L);
+    const bfp::Half4 h = bfp::split4(mantissa()), n = bfp::neg(h);
+    edge = fmaxl(edge, fabsl(val(n.h, 32) + n.l + val(h.h, 32) + h.l) * 0x1p-60L);
+  }
+  std::printf("edges %.3Lg\n", edge);
   Sum cr, rv, sm, ax;
   for (int i = 0; i < 100000; i++) {
     const double fa = std::exp(U(-20, 20)), fb = std::exp(U(-20, 20));

@@ -25,3 +25,6 @@ def test_operations_are_no_less_exact_than_fp64(tmp_path):
     for name in ("sin", "cos", "reciprocal", "rsqrt"):  # below a rounding of FP64 near 1
         assert got[name][0] <= 2.0**-53, (name, got[name])
     assert got["rounding"][0] <= 2.0**-53 * (1 + 1e-9)  # results are rounded once, to nearest
+    # halves at the ends of their range: two products, each off by the low product (2^-58 of the
+    # norms' 2^120) and a rounding (2^-57); a negated mantissa by one unit
+    assert got["edges"][0] <= 2.0**-55
