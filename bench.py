@@ -44,7 +44,7 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 KERNEL = "block floating point"
 KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39012326 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "b68f3c723a19196d60fa94897df9c9cb8f7b289f787c74717f921a1adf9db3ae"
+KERNEL_SOURCE_SHA256 = "4d9d5b52c492b99c9cb164803314ff517f4d4f9e519c242577f61c091df3ba1a"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

@@ -1,5 +1,6 @@
 // Launches of the block-floating-point sweep: environments per block.
 #include "bfp_launch.h"
+#include "bfp_diff.cuh"
 
 #include <map>
 #include <mutex>
@@ -54,6 +55,36 @@ cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const S
     case 16: return launch_bfp_step_e16(dm, ops, a, shape, s);
     case 32: return launch_bfp_step_e32(dm, ops, a, shape, s);
     default: return cudaErrorNotSupported;
+  }
+}
+
+#define SG_DIFF(E) \
+  cudaError_t launch_bfp_diff_e##E(BfpDiff, const DModel*, const RolloutArgs*, const VjpArgs*, const BlkShape&, cudaStream_t);
+SG_DIFF(4)
+SG_DIFF(8)
+SG_DIFF(16)
+SG_DIFF(32)
+#undef SG_DIFF
+
+int64_t bfp_record_doubles(const BfpTree& t) { return bfp::blk_record_doubles(t.nv, t.nq, t.npairs); }
+
+cudaError_t launch_bfp_diff(BfpDiff what, const DModel* dm, const BfpTree& t, const RolloutArgs* r, const VjpArgs* v,
+                            cudaStream_t s) {
+  const int64_t n = r ? r->n : v->n;
+  if (n <= 0) return cudaSuccess;
+  if (t.nv <= 0) return cudaErrorNotSupported;
+  // the reverse pass takes fewer environments per block than the sweeps before it, if any: both
+  // fit or neither is used
+  if (blk_shape(t, true, n).envs == 0) return cudaErrorNotSupported;
+  const bool adjoint = what == BfpDiff::reverse || what == BfpDiff::rnea_vjp || what == BfpDiff::aba_vjp;
+  const BlkShape shape = blk_shape(t, adjoint, what == BfpDiff::replay ? n * r->s_cnt : n);
+  BlkShape b = shape;
+  b.blocks = unsigned((n + b.envs - 1) / b.envs);
+  switch (b.envs) {
+    case 4: return launch_bfp_diff_e4(what, dm, r, v, b, s);
+    case 8: return launch_bfp_diff_e8(what, dm, r, v, b, s);
+    case 16: return launch_bfp_diff_e16(what, dm, r, v, b, s);
+    default: return launch_bfp_diff_e32(what, dm, r, v, b, s);
   }
 }
 

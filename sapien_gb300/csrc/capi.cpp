@@ -720,6 +720,11 @@ int sgdyn_compute_inverse_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(qdd_bar, n, nv, layout);
+    if (Mo.bfp_ok()) {
+      const cudaError_t e = launch_bfp_diff(BfpDiff::rnea_vjp, dm, bfp_tree(Mo), nullptr, &a,
+                                            static_cast<cudaStream_t>(stream));
+      if (e != cudaErrorNotSupported) return launch_status(e);
+    }
     std::string why;
     if (launch_vjp_jit(Mo, false, a, static_cast<cudaStream_t>(stream), &why)) return SGDYN_OK;
     return launch_status(launch_rnea_vjp(dm, Mo.njoints(), a, static_cast<cudaStream_t>(stream)));
@@ -751,6 +756,11 @@ int sgdyn_compute_forward_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(tau_bar, n, nv, layout);
+    if (Mo.bfp_ok()) {
+      const cudaError_t e = launch_bfp_diff(BfpDiff::aba_vjp, dm, bfp_tree(Mo), nullptr, &a,
+                                            static_cast<cudaStream_t>(stream));
+      if (e != cudaErrorNotSupported) return launch_status(e);
+    }
     std::string why;
     if (launch_vjp_jit(Mo, true, a, static_cast<cudaStream_t>(stream), &why)) return SGDYN_OK;
     return launch_status(launch_aba_vjp(dm, Mo.njoints(), a, static_cast<cudaStream_t>(stream)));
@@ -863,6 +873,10 @@ int sgdyn_rollout_forward(const sgdyn_model* m, int64_t n, int T, double dt, con
     a.qT = qT; a.qdT = qdT; a.q_ckpt = q_ckpt; a.qd_ckpt = qd_ckpt;
     std::string why;
     const auto st = static_cast<cudaStream_t>(stream);
+    if (Mo.bfp_ok() && g_rollout_lanes.load() == 0) {
+      const cudaError_t e = launch_bfp_diff(BfpDiff::rollout, dm, bfp_tree(Mo), &a, nullptr, st);
+      if (e != cudaErrorNotSupported) return launch_status(e);
+    }
     if (rollout_lanes(Mo, n) == 3) {
       if (launch_rollout3_jit(Mo, a, st, &why)) return SGDYN_OK;
       return launch_status(launch_rollout_forward3(dm, Mo.njoints(), a, st));
@@ -977,6 +991,17 @@ int sgdyn_rollout_backward(const sgdyn_model* m, int64_t n, int T, double dt, in
     a.q0_bar = q0_bar; a.qd0_bar = qd0_bar; a.tau_bar = tau_bar; a.scratch = scratch;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nj = Mo.njoints();
+    if (Mo.bfp_ok() && g_rollout_lanes.load() == 0 && T > 0) {
+      // its records are smaller than the intermediates the scratch is sized for
+      const BfpTree tree = bfp_tree(Mo);
+      const int64_t seg = bfp_record_doubles(tree) * checkpoint_every * n;
+      const auto run = [&](BfpDiff what) {
+        return [&, what](const RolloutArgs& g) { return launch_bfp_diff(what, dm, tree, &g, nullptr, st); };
+      };
+      const cudaError_t e =
+          rollout_backward_grouped(a, seg, scratch_bytes / 8, run(BfpDiff::replay), run(BfpDiff::reverse));
+      if (e != cudaErrorNotSupported) return launch_status(e);
+    }
     const int lanes = rollout_lanes(Mo, n);
     // two scratch halves of G segments each and at least two groups: overlap recompute and
     // reverse on two streams (not while the caller's stream is being captured)

@@ -115,6 +115,13 @@ struct BfpTree {
   int nj, nv, nq, npairs, tree_ints;
 };
 cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s);
+// The differentiation sweeps of bfp_diff.cuh, likewise: a whole rollout; the replay of a group of
+// checkpoint segments and its reverse pass; vector-Jacobian products (r or v as each needs).
+enum class BfpDiff { rollout, replay, reverse, rnea_vjp, aba_vjp };
+cudaError_t launch_bfp_diff(BfpDiff what, const DModel* dm, const BfpTree& t, const RolloutArgs* r, const VjpArgs* v,
+                            cudaStream_t s);
+// Doubles per environment and step of the replay's records.
+int64_t bfp_record_doubles(const BfpTree& t);
 // Forward dynamics alone with three lanes per environment (team3.cuh; one-DoF joints and a
 // free-flyer root).
 cudaError_t launch_aba3(const DModel* dm, int nj, const StepArgs& a, cudaStream_t s);

@@ -1,4 +1,4 @@
-"""The block-floating-point sweeps (csrc/bfp_block.cuh), which every batched
+"""The block-floating-point sweeps (csrc/bfp_block.cuh, csrc/bfp_diff.cuh), which every batched
 call takes with its settings automatic, against the oracle and against the FP64 sweeps that
 forced settings select. Sizes around the edges of their blocks (4 to 32 environments, fewer per
 block while there are few blocks), both layouts, and inputs that send single environments of a
@@ -133,3 +133,92 @@ def test_structure_of_arrays_equals_env_major(name, n):
                                 ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
     for k, o in zip(keys, outs):
         assert torch.equal(o.t().reshape(want[k].shape), want[k]), k
+
+
+@pytest.mark.parametrize("name,n", [("slide", 3), ("mixed", 37), ("arm9", 9), ("quadruped", 21), ("humanoid", 5)])
+def test_gradients_match_fp64(name, n):
+    """Vector-Jacobian products and a rollout over three checkpoint segments with its reverse
+    pass, against the FP64 kernels; the smallest scratch (a segment at a time) gives the same
+    bits as the largest."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    q, qd, qdd, tau = cuda(*robot.sample(n, seed=6))
+    T, K = 8, 3
+    taus = tau.unsqueeze(0).repeat(T, 1, 1).contiguous()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    qTb = torch.randn(n, pm.nq_ext, generator=g, dtype=torch.float64, device="cuda")
+    qdTb = torch.randn(n, pm.nv, generator=g, dtype=torch.float64, device="cuda")
+
+    def run():
+        qT, qdT, qc, qdc = AD.rollout_forward(pm, q, 0.1 * qd, taus, 1e-3, K)
+        back = [AD.rollout_backward(pm, qc, qdc, taus, 1e-3, K, qTb, qdTb, max_scratch_bytes=b) for b in (0, 1 << 30)]
+        for a, b in zip(*back):
+            assert torch.equal(a, b)
+        return [qT, qdT, qc, qdc, *back[0]]
+
+    mine = run()
+    with fp64_route():
+        want = run()
+    for i, (a, b) in enumerate(zip(mine, want)):
+        assert rel_per_env(a.cpu().numpy().reshape(-1, a.shape[-1]), b.cpu().numpy().reshape(-1, b.shape[-1])) <= 1e-9, i
+    # the products against a one-step central difference of the sweep along a random direction
+    d = [torch.randn(n, pm.nv, generator=g, dtype=torch.float64, device="cuda") for _ in range(2)]
+    w = qdTb
+    for vjp, call, x in ((AD.inverse_dynamics_vjp, pm.compute_inverse_dynamics_batched, qdd),
+                         (AD.forward_dynamics_vjp, pm.compute_forward_dynamics_batched, tau)):
+        _, vb, xb = vjp(pm, q, qd, x, w)
+        h = 1e-6
+        fd = ((call(q, qd + h * d[0], x + h * d[1]) - call(q, qd - h * d[0], x - h * d[1])) * w).sum(1) / (2 * h)
+        got = (vb * d[0]).sum(1) + (xb * d[1]).sum(1)
+        scale = (vb.abs() * d[0].abs()).sum(1) + (xb.abs() * d[1].abs()).sum(1)
+        assert float(((got - fd).abs() / scale).max()) <= 1e-6
+
+
+def test_rollout_that_leaves_the_range_matches_fp64():
+    """A rollout whose state overflows part way: the FP64 algebra repeats that environment from
+    its start; the others keep their bits."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS["arm9"]()
+    pm, _ = pair(robot)
+    n, T = 20, 4
+    q, qd, _, tau = robot.sample(n, seed=8)
+    taus = np.repeat(tau[None], T, axis=0)
+    ref = AD.rollout_forward(pm, *cuda(q, qd, taus), 1e-3, None)[:2]
+    taus[2, 7] = 1e70
+    mine = AD.rollout_forward(pm, *cuda(q, qd, taus), 1e-3, None)[:2]
+    with fp64_route():
+        want = AD.rollout_forward(pm, *cuda(q, qd, taus), 1e-3, None)[:2]
+    keep = [e for e in range(n) if e != 7]
+    for a, b, w in zip(mine, ref, want):
+        assert torch.equal(a[keep], b[keep])
+        assert np.isfinite(a[7].cpu().numpy()).all() == np.isfinite(w[7].cpu().numpy()).all()
+
+
+def test_reverse_pass_that_leaves_the_range_matches_fp64():
+    """An adjoint beyond the integer form's range, with one segment's scratch at a time: each
+    group's reverse pass goes on from the previous one's results in place."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS["arm9"]()
+    pm, _ = pair(robot)
+    n, T, K = 20, 8, 3
+    q, qd, _, tau = cuda(*robot.sample(n, seed=9))
+    taus = tau.unsqueeze(0).repeat(T, 1, 1).contiguous()
+    bars = [torch.ones(n, pm.nv, dtype=torch.float64, device="cuda") for _ in range(2)]
+    bars[0][7] *= 1e70
+    _, _, qc, qdc = AD.rollout_forward(pm, q, 0.1 * qd, taus, 1e-3, K)
+    mine = AD.rollout_backward(pm, qc, qdc, taus, 1e-3, K, *bars, max_scratch_bytes=0)
+    with fp64_route():
+        _, _, qc, qdc = AD.rollout_forward(pm, q, 0.1 * qd, taus, 1e-3, K)
+        want = AD.rollout_backward(pm, qc, qdc, taus, 1e-3, K, *bars, max_scratch_bytes=0)
+    for a, b in zip(mine, want):
+        assert rel_per_env(a.cpu().numpy().reshape(-1, a.shape[-1]), b.cpu().numpy().reshape(-1, b.shape[-1])) <= 1e-9
