@@ -25,6 +25,7 @@
 // 4215) issued at 34 % of the schedulers' rate, waiting at barriers and for instruction fetch.
 #pragma once
 #include "bfp.cuh"
+#include "se3.cuh"
 #include "step_kernel.cuh"
 
 // on lambdas: inlined even where they are called more than once, so that the block state they
@@ -634,6 +635,12 @@ __device__ __forceinline__ void blk_back(const Blk<A, E>& b) {
   }
 }
 
+// S_c . (subtree force of the column's joint)
+template <class A, int E>
+__device__ __forceinline__ double blk_torque(const Blk<A, E>& b, int c) {
+  return A::get(dot(b.S(c), b.frc(b.col_joint[c])));
+}
+
 // qdd (tree columns, at b + nv) = M^-1 (tau - bias) from the inputs in shared memory.
 template <class A, int E>
 __device__ __forceinline__ void blk_forward_dynamics(const Blk<A, E>& b) {
@@ -642,7 +649,7 @@ __device__ __forceinline__ void blk_forward_dynamics(const Blk<A, E>& b) {
   blk_motion_forces(b, false);
   blk_subtrees(b, true, true);
   if (b.col >= 0)
-    b.setD(b.L.b + b.col, b.tau(b.ext[b.col]) - A::get(dot(b.S(b.col), b.frc(b.col_joint[b.col]))));
+    b.setD(b.L.b + b.col, b.tau(b.ext[b.col]) - blk_torque(b, b.col));
   blk_mass_matrix(b, true, false);
   blk_solve(b);
 }
@@ -682,11 +689,33 @@ __device__ __forceinline__ void blk_load(const Blk<A, E>& b, int ops, const Step
   blk_check_quaternion(b);
 }
 
-// One sweep over the block's environments e0 .. e0 + envs - 1; results are written for those
-// with want(environment in block).
-template <class A, int E, class Want>
-__device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const StepArgs& args, int64_t e, int64_t e0, int envs,
-                                         const Want& want) {
+// Semi-implicit Euler in place on the environment's rows of q and qd (args.q, args.qd) from the
+// inputs in shared memory and qdd at b + nv, as hetero_integrate_kernel does it.
+template <class A, int E>
+__device__ __forceinline__ void blk_euler_rows(const Blk<A, E>& b, const StepArgs& args, int64_t e, double dt) {
+  if (!b.j) return;
+  const DJoint& J = b.J[b.j];
+  double v[6], q[7];
+  const int w = J.kind == JK_FREEFLYER ? 6 : 1;
+#pragma unroll 1
+  for (int k = 0; k < w; k++) {
+    v[k] = fma(dt, b.D(b.L.b + b.nv + J.ivx + k), b.qd(J.vcol + k));
+    stv(args.qd, e, J.vcol + k, v[k]);
+  }
+  if (J.kind == JK_FREEFLYER) {
+    for (int k = 0; k < 7; k++) q[k] = b.q(J.qcol + k);
+    free_flyer_step(q, v, dt);
+    for (int k = 0; k < 7; k++) stv(args.q, e, J.qcol + k, q[k]);
+  } else {
+    stv(args.q, e, J.qcol, fma(dt, v[0], b.q(J.qcol)));
+  }
+}
+
+// One sweep over the block's environments, rows row(0 .. envs - 1) of the arrays (this thread's:
+// e); results are written for those with want(environment in block).
+template <class A, int E, class Row, class Want>
+__device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const StepArgs& args, int64_t e, const Row& row,
+                                         int envs, const Want& want) {
   typedef typename A::Sc Sc;
   typedef typename A::Vec Vec;
   typedef typename A::Rot Rot;
@@ -737,7 +766,7 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
   if (kVel) blk_motion_forces(b, kRNEA && !kABA);
   blk_subtrees(b, kVel, kComposite);
   if (kVel && c >= 0) {
-    const double f = A::get(dot(b.S(c), b.frc(b.col_joint[c])));
+    const double f = blk_torque(b, c);
     if (kABA) b.setD(b.L.b + c, f);
     else if (valid) stv(args.tau_out, e, xc, f);
   }
@@ -755,7 +784,7 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
       const int i = b.pair_of[rc];
 #pragma unroll 1
       for (int el = 0; el < envs; el++)
-        if (want(el)) stv(args.M, e0 + el, rc, i < 0 ? 0.0 : __longlong_as_double(b.w[(b.L.Y + i) * E + el]));
+        if (want(el)) stv(args.M, row(el), rc, i < 0 ? 0.0 : __longlong_as_double(b.w[(b.L.Y + i) * E + el]));
     }
   }
   if (!kABA) return;
@@ -783,22 +812,47 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
 
 #ifdef __CUDACC__
 // (at most 640 threads, so that a thread may hold 96 registers)
-template <int E>
-__global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_block_kernel(const DModel* __restrict__ model, int ops, const StepArgs args) {
+// Runs body(block state, valid) in block floating point, and again in FP64 for the environments
+// that refused (valid then holds for those only).
+template <int E, class F>
+__device__ __forceinline__ void blk_run(const DModel* model, long long* smem, bool adjoint, int envs, const F& body) {
+  bfp::Blk<bfp::BfpAlg, E> b;
+  b.init(model, smem, adjoint);
+  if (b.slot == 0) b.X(b.L.ints - 1) = 0;
+  __syncthreads();
+  body(b, b.lane < envs);
+  __syncthreads();
+  const int refused = b.X(b.L.ints - 1);
+  if (__syncthreads_or(refused)) {
+    bfp::Blk<bfp::FpAlg, E> f;
+    f.init(model, smem, adjoint);
+    __syncthreads();
+    body(f, f.lane < envs && refused);
+  }
+}
+
+// ROWS: the environments are rows of the arrays by a list, and may take an Euler step (an
+// instantiation of its own: the plain sweep is 4 % slower with it).
+template <int E, bool ROWS>
+__global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_block_kernel(const DModel* __restrict__ model, int ops,
+                                                                        const StepArgs args, const BfpRows r) {
   extern __shared__ __align__(16) long long smem[];
   bfp::Blk<bfp::BfpAlg, E> b;
   b.init(model, smem);
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = args.n - e0 < E ? int(args.n - e0) : E;
-  const int64_t e = e0 + (b.lane < envs ? b.lane : envs - 1);
+  auto row = [&](int el) SG_INLINE { return ROWS ? int64_t(r.rows[e0 + el]) : e0 + el; };
+  const int64_t e = row(b.lane < envs ? b.lane : envs - 1);
   bfp::blk_load(b, ops, args, e);
-  bfp::blk_step(b, ops, args, e, e0, envs, [](int) { return true; });
+  bfp::blk_step(b, ops, args, e, row, envs, [](int) { return true; });
   const int refused = b.X(b.L.ints - 1);
+  if (ROWS && r.integrate && b.lane < envs && !refused) bfp::blk_euler_rows(b, args, e, r.dt);
   if (__syncthreads_or(refused)) {  // FP64 for the environments that the sweep above turned away
     bfp::Blk<bfp::FpAlg, E> f;
     f.init(model, smem);
     const int* flag = f.x + (f.L.ints - 1) * E;
-    bfp::blk_step(f, ops, args, e, e0, envs, [&](int lane) SG_INLINE { return flag[lane] != 0; });
+    bfp::blk_step(f, ops, args, e, row, envs, [&](int lane) SG_INLINE { return flag[lane] != 0; });
+    if (ROWS && r.integrate && f.lane < envs && refused) bfp::blk_euler_rows(f, args, e, r.dt);
   }
 }
 

@@ -30,8 +30,7 @@ namespace bfp {
 SG_HD int64_t blk_record_doubles(int nv, int nq, int npairs) { return nq + 2 * int64_t(nv) + npairs; }
 
 #ifdef __CUDACC__
-// (calls of their own: rare, long FP64 code whose registers the sweeps should not carry)
-static __device__ __noinline__ void ff_integrate(double* q, const double* d) { free_flyer_integrate(q, d); }
+// (a call of its own: rare, long FP64 code whose registers the sweeps should not carry)
 static __device__ __noinline__ void ff_integrate_adjoint(const double* d, double dt, double* g, double* vb) {
   Mot v{mk(vb[0], vb[1], vb[2]), mk(vb[3], vb[4], vb[5])};
   const Mot q = free_flyer_integrate_adjoint(Mot{mk(d[0], d[1], d[2]), mk(d[3], d[4], d[5])},
@@ -66,8 +65,8 @@ __device__ __forceinline__ void blk_integrate(const Blk<A, E>& b, double dt) {
     if (J.kind == JK_FREEFLYER) {
       double q[7], d[6];
       for (int k = 0; k < 7; k++) q[k] = b.q(J.qcol + k);
-      for (int k = 0; k < 6; k++) d[k] = dt * b.qd(J.vcol + k);
-      ff_integrate(q, d);
+      for (int k = 0; k < 6; k++) d[k] = b.qd(J.vcol + k);
+      free_flyer_step(q, d, dt);
       for (int k = 0; k < 7; k++) blk_in(b, J.qcol + k, q[k]);
     } else {
       blk_in(b, J.qcol, fma(dt, b.qd(J.vcol), b.q(J.qcol)));
@@ -349,25 +348,6 @@ __device__ __forceinline__ void blk_reverse(const Blk<A, E>& b, const RolloutArg
 }  // namespace bfp
 
 #ifdef __CUDACC__
-// Runs body(block state, valid) in block floating point, and again in FP64 for the environments
-// that refused (valid then holds for those only).
-template <int E, class F>
-__device__ __forceinline__ void blk_run(const DModel* model, long long* smem, bool adjoint, int envs, const F& body) {
-  bfp::Blk<bfp::BfpAlg, E> b;
-  b.init(model, smem, adjoint);
-  if (b.slot == 0) b.X(b.L.ints - 1) = 0;
-  __syncthreads();
-  body(b, b.lane < envs);
-  __syncthreads();
-  const int refused = b.X(b.L.ints - 1);
-  if (__syncthreads_or(refused)) {
-    bfp::Blk<bfp::FpAlg, E> f;
-    f.init(model, smem, adjoint);
-    __syncthreads();
-    body(f, f.lane < envs && refused);
-  }
-}
-
 template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_rollout_kernel(const DModel* __restrict__ model,
                                                                          const RolloutArgs a) {

@@ -40,20 +40,26 @@ BlkShape blk_shape(const BfpTree& t, bool adjoint, int64_t n) {
   return s;
 }
 
-cudaError_t launch_bfp_step_e4(const DModel*, int, const StepArgs&, const BlkShape&, cudaStream_t);
-cudaError_t launch_bfp_step_e8(const DModel*, int, const StepArgs&, const BlkShape&, cudaStream_t);
-cudaError_t launch_bfp_step_e16(const DModel*, int, const StepArgs&, const BlkShape&, cudaStream_t);
-cudaError_t launch_bfp_step_e32(const DModel*, int, const StepArgs&, const BlkShape&, cudaStream_t);
+#define SG_STEP(E)                                                                                             \
+  cudaError_t launch_bfp_step_e##E(const DModel*, int, const StepArgs&, const BfpRows&, const BlkShape&, cudaStream_t);
+SG_STEP(4)
+SG_STEP(8)
+SG_STEP(16)
+SG_STEP(32)
+#undef SG_STEP
 
-cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s) {
+bool bfp_step_fits(const BfpTree& t) { return t.nv > 0 && blk_shape(t, false, 1).envs > 0; }
+
+cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s,
+                            const BfpRows& r) {
   if (a.n <= 0) return cudaSuccess;
   if (t.nv <= 0) return cudaErrorNotSupported;
-  const BlkShape shape = blk_shape(t, false, a.n);
-  switch (shape.envs) {
-    case 4: return launch_bfp_step_e4(dm, ops, a, shape, s);
-    case 8: return launch_bfp_step_e8(dm, ops, a, shape, s);
-    case 16: return launch_bfp_step_e16(dm, ops, a, shape, s);
-    case 32: return launch_bfp_step_e32(dm, ops, a, shape, s);
+  const BlkShape b = blk_shape(t, false, a.n);
+  switch (b.envs) {
+    case 4: return launch_bfp_step_e4(dm, ops, a, r, b, s);
+    case 8: return launch_bfp_step_e8(dm, ops, a, r, b, s);
+    case 16: return launch_bfp_step_e16(dm, ops, a, r, b, s);
+    case 32: return launch_bfp_step_e32(dm, ops, a, r, b, s);
     default: return cudaErrorNotSupported;
   }
 }

@@ -148,6 +148,13 @@ int rollout_lanes(const Model& M, int64_t n) {
 
 }  // namespace
 
+bool fp64_forced() {
+  int fd = 0;
+  fd_method(-1, &fd);
+  return g_split_mode.load() != 2 || fd != 0;
+}
+
+
 // Lanes per environment of the rollout kernels for this model and batch (1 or 3).
 int rollout_lanes_for(const Model& M, int64_t n) { return rollout_lanes(M, n); }
 
@@ -225,9 +232,7 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
   // With every setting automatic: the block-floating-point sweep, one launch for any op set and
   // batch size (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings
   // (lanes, split, forward-dynamics route) and what that sweep cannot hold.
-  int fd_mode = 0;
-  fd_method(-1, &fd_mode);
-  if (Mo.bfp_ok() && Mo.lanes == 0 && g_split_mode.load() == 2 && fd_mode == 0 &&
+  if (Mo.bfp_ok() && Mo.lanes == 0 && !fp64_forced() &&
       !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
     const cudaError_t e = launch_bfp_step(dm, bfp_tree(Mo), ops, a, s);
     if (e == cudaSuccess) return SGDYN_OK;

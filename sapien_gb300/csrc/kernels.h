@@ -32,6 +32,14 @@ struct StepArgs {
   Arr poses, J, M, tau_out, qdd_out;    // outputs (p == nullptr when not requested)
 };
 
+// The rows of the arrays that a block sweep works on (null: 0 .. n - 1, and no Euler step), and
+// whether each environment then makes a semi-implicit Euler step of its q and qd, in place.
+struct BfpRows {
+  const int* rows = nullptr;
+  int integrate = 0;
+  double dt = 0.0;
+};
+
 struct LinkJacArgs {
   int64_t n;
   int link, local;
@@ -114,7 +122,13 @@ cudaError_t launch_step(const DModel* dm, int nj, int ops, const StepArgs& a, cu
 struct BfpTree {
   int nj, nv, nq, npairs, tree_ints;
 };
-cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s);
+cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const StepArgs& a, cudaStream_t s,
+                            const BfpRows& rows = {});
+// Whether a process-wide setting of the FP64 sweeps (step splitting, forward-dynamics method) is
+// other than automatic: they then run.
+bool fp64_forced();
+// Whether launch_bfp_step can hold the model.
+bool bfp_step_fits(const BfpTree& t);
 // The differentiation sweeps of bfp_diff.cuh, likewise: a whole rollout; the replay of a group of
 // checkpoint segments and its reverse pass; vector-Jacobian products (r or v as each needs).
 enum class BfpDiff { rollout, replay, reverse, rnea_vjp, aba_vjp };

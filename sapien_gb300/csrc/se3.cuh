@@ -170,6 +170,19 @@ SG_HD void free_flyer_integrate(double* q, const double* v) {
   q[6] = s * qw[0];
 }
 
+// q advanced by the twist dt qd. On the device a call of its own, so that every kernel that
+// integrates a free flyer contracts the same products and gives the same bits.
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+static __host__ __device__ __noinline__
+#else
+inline
+#endif
+void free_flyer_step(double* q, const double* qd, double dt) {
+  double v[6];
+  for (int k = 0; k < 6; k++) v[k] = dt * qd[k];
+  free_flyer_integrate(q, v);
+}
+
 // Semi-implicit Euler on one environment's rows: qd += dt qdd, then q advanced by dt qd
 // (angles and slides add; a free flyer moves on SE(3) by its body twist dt qd).
 template <class Tab>
@@ -178,14 +191,9 @@ SG_HD void integrate_env_t(const Tab& T, double* q, double* qd, const double* qd
   for (int i = 1; i < T.nj(); i++) {
     const DJoint& J = T.joint(i);
     if (J.kind == JK_FREEFLYER) {
-      double v[6];
 #pragma unroll
-      for (int k = 0; k < 6; k++) {
-        const double w = fma(dt, qdd[J.vcol + k], qd[J.vcol + k]);
-        qd[J.vcol + k] = w;
-        v[k] = dt * w;
-      }
-      free_flyer_integrate(q + J.qcol, v);
+      for (int k = 0; k < 6; k++) qd[J.vcol + k] = fma(dt, qdd[J.vcol + k], qd[J.vcol + k]);
+      free_flyer_step(q + J.qcol, qd + J.vcol, dt);
     } else {
       const double w = fma(dt, qdd[J.vcol], qd[J.vcol]);
       qd[J.vcol] = w;

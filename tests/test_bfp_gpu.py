@@ -222,3 +222,37 @@ def test_reverse_pass_that_leaves_the_range_matches_fp64():
         want = AD.rollout_backward(pm, qc, qdc, taus, 1e-3, K, *bars, max_scratch_bytes=0)
     for a, b in zip(mine, want):
         assert rel_per_env(a.cpu().numpy().reshape(-1, a.shape[-1]), b.cpu().numpy().reshape(-1, b.shape[-1])) <= 1e-9
+
+
+def test_mixed_batch_matches_fp64():
+    """One launch per model on its rows of the padded arrays, with and without the Euler step,
+    against the persistent FP64 kernel that a forced forward-dynamics method selects."""
+    import torch
+
+    from sapien_gb300.hetero import HeteroBatch
+
+    robots, moe = syn.hetero_mix(83, seed=3)
+    robots.append(ROBOTS["mixed"]())  # a model that no environment uses
+    batch = HeteroBatch([pair(r)[0] for r in robots], moe)
+    ins = [r.sample(int((moe == k).sum()), seed=k) for k, r in enumerate(robots)]
+    q, qd, qdd, tau = (f([x[i] for x in ins]) for i, f in enumerate((batch.pad_q, batch.pad_v, batch.pad_v, batch.pad_v)))
+    q[5, 0] = float("nan")  # its environment alone
+    ops = N.OP_MASS_MATRIX | N.OP_INVERSE_DYNAMICS | N.OP_FORWARD_DYNAMICS
+
+    def run():
+        out = {k: v.zero_() for k, v in batch.alloc_outputs(ops).items()}
+        batch.step(q, qd, qdd, tau, ops, out)
+        q1, qd1 = q.clone(), qd.clone()
+        acc = batch.alloc_outputs(N.OP_FORWARD_DYNAMICS)
+        batch.rollout_step(q1, qd1, tau, 1e-3, acc)
+        torch.cuda.synchronize()
+        return [out["mass_matrix"], out["qf"], out["qacc"], q1, qd1]
+
+    mine = run()
+    with fp64_route():
+        want = run()
+    keep = [e for e in range(len(moe)) if e != 5]
+    for a, b in zip(mine, want):
+        a, b = a.cpu().numpy().reshape(len(moe), -1), b.cpu().numpy().reshape(len(moe), -1)
+        assert rel_per_env(a[keep], b[keep]) <= 1e-9
+        assert not np.isfinite(a[5]).all() and not np.isfinite(b[5]).all()
