@@ -44,7 +44,7 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 KERNEL = "block floating point"
 KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39012326 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "80e6ae0f57a002fc21714935e24741474a03ef8f646022c3e50095b7872eb3d9"
+KERNEL_SOURCE_SHA256 = "bcff45712c68744e49ce92bb793fbc39cf97ca6f36527ab575456a2115cb5b18"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

@@ -856,6 +856,31 @@ __global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_block_kernel(const DM
   }
 }
 
+// PhysxArticulation::computePassiveForce on float32 state rows (physx_interop.cu): RNEA at zero
+// acceleration with the gravity and / or velocity terms.
+template <int E>
+__global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_passive_kernel(const DModel* __restrict__ model,
+                                                                          const PassiveArgs a) {
+  extern __shared__ __align__(16) long long smem[];
+  const int64_t e0 = int64_t(blockIdx.x) * E;
+  const int envs = a.n - e0 < E ? int(a.n - e0) : E;
+  blk_run<E>(model, smem, false, envs, [&](auto& b, bool valid) SG_INLINE {
+    const int64_t e = e0 + min(b.lane, envs - 1);
+    if (!a.gravity) b.g[0] = b.g[1] = b.g[2] = 0.0;
+    if (b.col >= 0) {  // one-DoF joints only: as many coordinates as columns
+      bfp::blk_in(b, b.col, double(a.qpos[e * a.in_stride + b.col]));
+      bfp::blk_in(b, b.nq + b.col, a.coriolis ? double(a.qvel[e * a.in_stride + b.col]) : 0.0);
+    }
+    __syncthreads();
+    bfp::blk_poses(b);
+    bfp::blk_columns(b, true);
+    bfp::blk_motion_forces(b, false);
+    bfp::blk_subtrees(b, true, false);
+    if (b.col >= 0 && valid)
+      a.qf[e * a.out_stride + b.ext[b.col]] = float(bfp::blk_torque(b, b.col));
+  });
+}
+
 // Launches a kernel with `smem` bytes of dynamic shared memory.
 template <class... P, class... Q>
 cudaError_t launch_block(void (*kernel)(P...), dim3 blocks, unsigned threads, size_t smem, cudaStream_t s,

@@ -7,4 +7,8 @@ cudaError_t launch_bfp_step_e16(const DModel* dm, int ops, const StepArgs& a, co
                                 cudaStream_t s) {
   return launch_block(r.rows ? bfp_block_kernel<16, true> : bfp_block_kernel<16, false>, b.blocks, b.threads, b.smem, s, dm, ops, a, r);
 }
+cudaError_t launch_bfp_passive_e16(const DModel* dm, const PassiveArgs& a, const BlkShape& b, cudaStream_t s) {
+  return launch_block(bfp_passive_kernel<16>, b.blocks, b.threads, b.smem, s, dm, a);
+}
+
 }  // namespace sgdyn

@@ -7,4 +7,8 @@ cudaError_t launch_bfp_step_e8(const DModel* dm, int ops, const StepArgs& a, con
                                 cudaStream_t s) {
   return launch_block(r.rows ? bfp_block_kernel<8, true> : bfp_block_kernel<8, false>, b.blocks, b.threads, b.smem, s, dm, ops, a, r);
 }
+cudaError_t launch_bfp_passive_e8(const DModel* dm, const PassiveArgs& a, const BlkShape& b, cudaStream_t s) {
+  return launch_block(bfp_passive_kernel<8>, b.blocks, b.threads, b.smem, s, dm, a);
+}
+
 }  // namespace sgdyn

@@ -41,7 +41,8 @@ BlkShape blk_shape(const BfpTree& t, bool adjoint, int64_t n) {
 }
 
 #define SG_STEP(E)                                                                                             \
-  cudaError_t launch_bfp_step_e##E(const DModel*, int, const StepArgs&, const BfpRows&, const BlkShape&, cudaStream_t);
+  cudaError_t launch_bfp_step_e##E(const DModel*, int, const StepArgs&, const BfpRows&, const BlkShape&, cudaStream_t); \
+  cudaError_t launch_bfp_passive_e##E(const DModel*, const PassiveArgs&, const BlkShape&, cudaStream_t);
 SG_STEP(4)
 SG_STEP(8)
 SG_STEP(16)
@@ -60,6 +61,19 @@ cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const S
     case 8: return launch_bfp_step_e8(dm, ops, a, r, b, s);
     case 16: return launch_bfp_step_e16(dm, ops, a, r, b, s);
     case 32: return launch_bfp_step_e32(dm, ops, a, r, b, s);
+    default: return cudaErrorNotSupported;
+  }
+}
+
+cudaError_t launch_bfp_passive(const DModel* dm, const BfpTree& t, const PassiveArgs& a, cudaStream_t s) {
+  if (a.n <= 0) return cudaSuccess;
+  if (t.nv <= 0) return cudaErrorNotSupported;
+  const BlkShape b = blk_shape(t, false, a.n);
+  switch (b.envs) {
+    case 4: return launch_bfp_passive_e4(dm, a, b, s);
+    case 8: return launch_bfp_passive_e8(dm, a, b, s);
+    case 16: return launch_bfp_passive_e16(dm, a, b, s);
+    case 32: return launch_bfp_passive_e32(dm, a, b, s);
     default: return cudaErrorNotSupported;
   }
 }

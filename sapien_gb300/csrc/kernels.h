@@ -40,6 +40,17 @@ struct BfpRows {
   double dt = 0.0;
 };
 
+// Passive forces on float32 state rows.
+struct PassiveArgs {
+  int64_t n;
+  const float* qpos;
+  const float* qvel;
+  int64_t in_stride;
+  float* qf;
+  int64_t out_stride;
+  int gravity, coriolis;
+};
+
 struct LinkJacArgs {
   int64_t n;
   int link, local;
@@ -129,6 +140,7 @@ cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const S
 bool fp64_forced();
 // Whether launch_bfp_step can hold the model.
 bool bfp_step_fits(const BfpTree& t);
+cudaError_t launch_bfp_passive(const DModel* dm, const BfpTree& t, const PassiveArgs& a, cudaStream_t s);
 // The differentiation sweeps of bfp_diff.cuh, likewise: a whole rollout; the replay of a group of
 // checkpoint segments and its reverse pass; vector-Jacobian products (r or v as each needs).
 enum class BfpDiff { rollout, replay, reverse, rnea_vjp, aba_vjp };

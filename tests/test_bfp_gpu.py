@@ -256,3 +256,35 @@ def test_mixed_batch_matches_fp64():
         a, b = a.cpu().numpy().reshape(len(moe), -1), b.cpu().numpy().reshape(len(moe), -1)
         assert rel_per_env(a[keep], b[keep]) <= 1e-9
         assert not np.isfinite(a[5]).all() and not np.isfinite(b[5]).all()
+
+
+@pytest.mark.parametrize("name,n", [("slide", 1), ("mixed", 35), ("arm9", 300), ("chain40", 6)])
+def test_passive_force_matches_fp64(name, n):
+    """Gravity and velocity terms on float32 rows with a gap between them, one environment with a
+    value that is not finite: the FP64 algebra's bits to a rounding of float32."""
+    import torch
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    q, qd, _, _ = robot.sample(n, seed=4)
+    rows = np.full((2, n, pm.nv + 3), 7.0, dtype=np.float32)
+    rows[0, :, : pm.nv], rows[1, :, : pm.nv] = q, qd
+    bad = n // 2 if n > 1 else None
+    if bad is not None:
+        rows[0, bad, 0] = np.inf
+    x, v = cuda(rows[0], rows[1])
+    wide = [torch.from_numpy(r[:, : pm.nv].astype(np.float64)).cuda() for r in rows]
+    zero = torch.zeros_like(wide[0])
+    pm0 = PinocchioModel(robot.urdf, [0, 0, 0])
+    pm0.set_joint_order(robot.joint_names)
+    with fp64_route():
+        full = pm.compute_inverse_dynamics_batched(wide[0], wide[1], zero)
+        still = pm.compute_inverse_dynamics_batched(wide[0], zero, zero)
+        free = pm0.compute_inverse_dynamics_batched(wide[0], wide[1], zero)
+    for gravity, coriolis, want in ((True, True, full), (True, False, still), (False, True, free)):
+        got = pm.compute_passive_force_batched(x, v, gravity=gravity, coriolis_and_centrifugal=coriolis)
+        got, want = got.cpu().numpy()[:, : pm.nv], want.cpu().numpy()
+        keep = [e for e in range(n) if e != bad]
+        assert rel_per_env(got[keep].astype(np.float64), want[keep]) <= 2.0**-23
+        if bad is not None:
+            assert not np.isfinite(got[bad]).all()
