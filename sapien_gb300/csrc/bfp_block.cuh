@@ -18,9 +18,9 @@
 //
 // Measured (GB300, device time per call; before: the FP64 sweeps, specialised per model or in
 // teams of lanes, that still serve forced settings and models out of range). All five ops: 7-DoF
-// arm, 16 environments 143 -> 32 us, 1000: 145 -> 36 us; 9-DoF arm, 16384: 156 -> 96 us. CRBA +
-// RNEA + forward dynamics: 9-DoF arm, 131071: 792 -> 544 us; 35-DoF humanoid, 1024: 422 -> 78 us.
-// Forward dynamics alone, 18-DoF quadruped, 3001: 84 -> 43 us. What bounds it at 16384 9-DoF
+// arm, 16 environments 143 -> 32 us, 1000: 145 -> 33 us; 9-DoF arm, 16384: 156 -> 96 us. CRBA +
+// RNEA + forward dynamics: 9-DoF arm, 131071: 792 -> 544 us; 35-DoF humanoid, 1024: 422 -> 68 us.
+// Forward dynamics alone, 18-DoF quadruped, 3001: 84 -> 41 us. What bounds it at 16384 9-DoF
 // arms: 2381 warp instructions per environment (170 of its thread instructions in FP64, before
 // 4215) issued at 34 % of the schedulers' rate, waiting at barriers and for instruction fetch.
 #pragma once
@@ -572,9 +572,11 @@ __device__ __forceinline__ void blk_pivot(const Blk<A, E>& b, int a, int diag) {
 }
 template <class A, int E>
 __device__ __forceinline__ void blk_back(const Blk<A, E>& b);
-// M = L^T D L with the right-hand side in b carried along, then x = M^-1 b (after b). Column by
-// column, slot c updates row c if c is an ancestor of the column: f = h / D, then h_cd -= f h_ad
-// along the row. L's entries go to S / V in FP64; the slot of the next column leaves its pivot.
+// M = L^T D L with the right-hand side in b carried along, then x = M^-1 b (after b). By levels
+// from the deepest columns, all columns of a level between two barriers (column by column, with
+// nv of them, 8192 35-DoF humanoids took 366 us instead of 297): slot c updates row c for every
+// column a of the level that it is an ancestor of, f = h / D, then h_cd -= f h_ad along the row;
+// the slots one level up then leave their pivots. L's entries go to S / V in FP64.
 // Then L x = D^-1 y by levels, one product per column and level. M is in A: scaled fixed point
 // (M_ac = h_ac 2^(s_a + s_c - 60) with |h| <= 2^60, the scales from the diagonal: a positive
 // definite matrix has |M_ac| <= sqrt(M_aa M_cc), and so have the matrices that elimination
@@ -582,16 +584,19 @@ __device__ __forceinline__ void blk_back(const Blk<A, E>& b);
 // L_ac = f 2^(x_a + s_c - s_a)), or FP64.
 template <class A, int E>
 __device__ __forceinline__ void blk_solve(const Blk<A, E>& b) {
-  const int nv = b.nv;
-  if (b.slot == nv - 1) blk_pivot(b, nv - 1, b.L.A + b.row_start[nv - 1] + b.depth[nv - 1]);
+  const int nv = b.nv, col = b.col;
+  const int row = col >= 0 ? b.L.A + b.row_start[col] : 0, dr = col >= 0 ? b.depth[col] : nv;
+  if (dr == b.col_levels - 1) blk_pivot(b, col, row + dr);
   __syncthreads();
-  const int col = b.col, row = col >= 0 ? b.L.A + b.row_start[col] : 0, dr = col >= 0 ? b.depth[col] : 0;
 #pragma unroll 1
-  for (int a = nv - 1; a >= 0; a--) {
-    const int da = b.depth[a], ra = b.row_start[a], h0 = b.L.A + ra;
-    const double ba = b.D(b.L.b + a);
-    if (col >= 0 && col < a) {
-      if (dr < da && b.pair_col[ra + dr] == col) {  // an ancestor of column a
+  for (int da = b.col_levels - 1; da >= 0; da--) {
+    if (dr < da) {  // columns of depth da are final: their ancestors take them
+      const int hi = b.col_level_start[da + 1];
+#pragma unroll 1
+      for (int k = b.col_level_start[da]; k < hi; k++) {
+        const int a = b.col_order[k], ra = b.row_start[a], h0 = b.L.A + ra;
+        if (b.pair_col[ra + dr] != col) continue;
+        const double ba = b.D(b.L.b + a);
         if constexpr (A::kFixed) {
           const int xa = b.X(b.L.xs + nv + a);
           const Half4 f = split4(mul60(split4(shl(b.W(h0 + dr), xa)), split4(b.W(h0 + da))));
@@ -608,12 +613,12 @@ __device__ __forceinline__ void blk_solve(const Blk<A, E>& b) {
           b.setD(b.L.b + col, fma(-f, ba, b.D(b.L.b + col)));
         }
       }
-      if (col == a - 1) blk_pivot(b, a - 1, row + dr);
-    } else if (col == a) {
+      if (dr == da - 1) blk_pivot(b, col, row + dr);
+    } else if (dr == da) {
       double dinv;
-      if constexpr (A::kFixed) dinv = to_double(b.W(h0 + da), 2 * b.X(b.L.xs + nv + a) - 58 - 2 * b.X(b.L.xs + a));
-      else dinv = b.D(h0 + da);
-      b.setD(b.L.b + nv + a, ba * dinv);
+      if constexpr (A::kFixed) dinv = to_double(b.W(row + dr), 2 * b.X(b.L.xs + nv + col) - 58 - 2 * b.X(b.L.xs + col));
+      else dinv = b.D(row + dr);
+      b.setD(b.L.b + nv + col, b.D(b.L.b + col) * dinv);
     }
     __syncthreads();
   }
