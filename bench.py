@@ -44,7 +44,7 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 KERNEL = "block floating point"
 KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39004134 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "21107225e753807c9dd5f9e31e19328b5c9f99106f39e07231777ae8e6fde50d"
+KERNEL_SOURCE_SHA256 = "3d0f82662d115f25457d8c0e34f2ba9d184bb41b9c92bbfe79a35e79109b18f4"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

@@ -1,5 +1,5 @@
 // Instantiations of the link-Jacobian, Coriolis and IK kernels for trees of up to 64 joints.
-#include "aux_kernels.cuh"
+#include "bfp_ik.cuh"
 
 namespace sgdyn {
 
@@ -11,11 +11,8 @@ cudaError_t launch_coriolis_j64(const DModel* dm, const CoriolisArgs& a, cudaStr
   coriolis_kernel<64><<<unsigned((a.n + 31) / 32), 32, 0, s>>>(dm, a);
   return cudaGetLastError();
 }
-cudaError_t launch_ik_j64(const DModel* dm, const IkArgs& a, cudaStream_t s) {
-  static int occ = 0;
-  if (occ == 0 && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ik_kernel<64>, 32, 0) != cudaSuccess) occ = 1;
-  ik_kernel<64><<<balanced_grid(a.n, occ), 32, 0, s>>>(dm, a);
-  return cudaGetLastError();
+cudaError_t launch_ik_j64(const DModel* dm, const IkArgs& a, bool fixed, cudaStream_t s) {
+  return launch_ik_kernel(fixed ? bfp_ik_kernel<64> : ik_kernel<64>, dm, a, s);
 }
 
 }  // namespace sgdyn

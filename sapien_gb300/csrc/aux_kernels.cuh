@@ -204,6 +204,13 @@ inline unsigned balanced_grid(int64_t n, int blocks_per_sm) {
   const int64_t rounds = (blocks + cap - 1) / cap;
   return unsigned(rounds > 0 ? (blocks + rounds - 1) / rounds : 1);
 }
+template <class K>
+cudaError_t launch_ik_kernel(K* kernel, const DModel* dm, const IkArgs& a, cudaStream_t s) {
+  int occ = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, 32, 0) != cudaSuccess) occ = 1;
+  kernel<<<balanced_grid(a.n, occ), 32, 0, s>>>(dm, a);
+  return cudaGetLastError();
+}
 #endif
 
 // computeInverseKinematics (pinocchio_model.cpp:228-300): damped-least-squares CLIK on the

@@ -694,7 +694,7 @@ int sgdyn_compute_inverse_kinematics(const sgdyn_model* m, int64_t n, int link, 
     a.err = make_arr(err_out, n, 6, layout);
     a.mask = mask;
     a.success = success;
-    cudaError_t e = launch_ik(dm, Mo.njoints(), a, static_cast<cudaStream_t>(stream));
+    cudaError_t e = launch_ik(dm, Mo.njoints(), a, Mo.bfp_ok() && !fp64_forced(), static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(SGDYN_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString(e));
     return SGDYN_OK;
   });

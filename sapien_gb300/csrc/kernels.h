@@ -156,7 +156,8 @@ cudaError_t launch_step_team(const DModel* dm, int nj, const int* team, int lane
                              cudaStream_t s);
 cudaError_t launch_link_jacobian(const DModel* dm, int nj, const LinkJacArgs& a, cudaStream_t s);
 cudaError_t launch_coriolis(const DModel* dm, int nj, const CoriolisArgs& a, cudaStream_t s);
-cudaError_t launch_ik(const DModel* dm, int nj, const IkArgs& a, cudaStream_t s);
+// fixed: in block floating point (bfp_ik.cuh; the model has to fit it)
+cudaError_t launch_ik(const DModel* dm, int nj, const IkArgs& a, bool fixed, cudaStream_t s);
 cudaError_t launch_rnea_vjp(const DModel* dm, int nj, const VjpArgs& a, cudaStream_t s);
 cudaError_t launch_aba_vjp(const DModel* dm, int nj, const VjpArgs& a, cudaStream_t s);
 cudaError_t launch_fk_vjp(const DModel* dm, int nj, const FkVjpArgs& a, cudaStream_t s);

@@ -42,7 +42,7 @@ namespace sgdyn {
 #define SG_DECL(J)                                                                    \
   cudaError_t launch_link_jacobian_j##J(const DModel*, const LinkJacArgs&, cudaStream_t); \
   cudaError_t launch_coriolis_j##J(const DModel*, const CoriolisArgs&, cudaStream_t);    \
-  cudaError_t launch_ik_j##J(const DModel*, const IkArgs&, cudaStream_t);
+  cudaError_t launch_ik_j##J(const DModel*, const IkArgs&, bool, cudaStream_t);
 SG_DECL(16)
 SG_DECL(32)
 SG_DECL(64)
@@ -66,12 +66,12 @@ cudaError_t launch_coriolis(const DModel* dm, int nj, const CoriolisArgs& a, cud
     default: return cudaErrorInvalidValue;
   }
 }
-cudaError_t launch_ik(const DModel* dm, int nj, const IkArgs& a, cudaStream_t s) {
+cudaError_t launch_ik(const DModel* dm, int nj, const IkArgs& a, bool fixed, cudaStream_t s) {
   if (a.n <= 0) return cudaSuccess;
   switch (stash_bucket(nj)) {
-    case 16: return launch_ik_j16(dm, a, s);
-    case 32: return launch_ik_j32(dm, a, s);
-    case 64: return launch_ik_j64(dm, a, s);
+    case 16: return launch_ik_j16(dm, a, fixed, s);
+    case 32: return launch_ik_j32(dm, a, fixed, s);
+    case 64: return launch_ik_j64(dm, a, fixed, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -288,3 +288,39 @@ def test_passive_force_matches_fp64(name, n):
         assert rel_per_env(got[keep].astype(np.float64), want[keep]) <= 2.0**-23
         if bad is not None:
             assert not np.isfinite(got[bad]).all()
+
+
+@pytest.mark.parametrize("name,n,steps", [("slide", 2, 3), ("mixed", 70, 6), ("arm9", 33, 6), ("quadruped", 5, 2),
+                                          ("chain40", 3, 2)])
+def test_inverse_kinematics_matches_fp64(name, n, steps):
+    """A few iterations towards another pose, free and with a joint held, one environment with a
+    target that is not finite, and no iteration at all (the start's own error)."""
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    q0, _, _, _ = robot.sample(n, seed=3)
+    link = len(robot.link_names) - 1
+    ahead = pm.step_batched(*cuda(*robot.sample(n, seed=5)), ops=N.OP_FK)["link_poses"]
+    target = ahead.cpu().numpy().reshape(n, -1, 7)[:, link].copy()
+    if n > 2:
+        target[1, 0] = np.nan
+    mask = np.ones(pm.nv, dtype=np.int32)
+    mask[-1] = 0
+    start, goal = cuda(q0, target)
+
+    def run():
+        out = []
+        for m, it in ((None, steps), (mask, steps), (None, 0)):
+            q, ok, err = pm.compute_inverse_kinematics_batched(link, goal, start, max_iterations=it, active_qmask=m)
+            out += [q.cpu().numpy(), ok.cpu().numpy(), err.cpu().numpy()]
+        return out
+
+    mine = run()
+    with fp64_route():
+        want = run()
+    keep = [e for e in range(n) if np.isfinite(target[e]).all()]
+    for i, (a, b) in enumerate(zip(mine, want)):
+        if i % 3 == 1:
+            assert (a == b).all()
+        else:
+            assert rel_per_env(a[keep], b[keep]) <= 1e-9
+            assert (np.isfinite(a) == np.isfinite(b)).all()
