@@ -12,7 +12,7 @@ cudaError_t launch_coriolis_j32(const DModel* dm, const CoriolisArgs& a, cudaStr
   return cudaGetLastError();
 }
 cudaError_t launch_ik_j32(const DModel* dm, const IkArgs& a, bool fixed, cudaStream_t s) {
-  return launch_ik_kernel(fixed ? bfp_ik_kernel<32> : ik_kernel<32>, dm, a, s);
+  return fixed ? launch_bfp_ik<32>(dm, a, s) : launch_ik_kernel(ik_kernel<32>, dm, a, s);
 }
 
 }  // namespace sgdyn

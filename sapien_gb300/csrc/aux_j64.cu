@@ -12,7 +12,7 @@ cudaError_t launch_coriolis_j64(const DModel* dm, const CoriolisArgs& a, cudaStr
   return cudaGetLastError();
 }
 cudaError_t launch_ik_j64(const DModel* dm, const IkArgs& a, bool fixed, cudaStream_t s) {
-  return launch_ik_kernel(fixed ? bfp_ik_kernel<64> : ik_kernel<64>, dm, a, s);
+  return fixed ? launch_bfp_ik<64>(dm, a, s) : launch_ik_kernel(ik_kernel<64>, dm, a, s);
 }
 
 }  // namespace sgdyn

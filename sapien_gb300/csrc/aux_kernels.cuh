@@ -192,15 +192,15 @@ __global__ void __launch_bounds__(32) coriolis_kernel(const DModel* __restrict__
 // (occupancy x SMs) allows, with the environments spread evenly over the rounds. Without
 // it, a batch slightly above one wave (65536 CLIK solves: 2048 warps for ~1800 resident)
 // runs a second, nearly empty wave at full per-warp latency.
+inline int multiprocessors() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
+    return 1;
+  return sms;
+}
 inline unsigned balanced_grid(int64_t n, int blocks_per_sm) {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (sms <= 0) sms = 1;
-  }
-  const int64_t blocks = (n + 31) / 32, cap = int64_t(sms) * (blocks_per_sm > 0 ? blocks_per_sm : 1);
+  const int64_t blocks = (n + 31) / 32, cap = int64_t(multiprocessors()) * (blocks_per_sm > 0 ? blocks_per_sm : 1);
   const int64_t rounds = (blocks + cap - 1) / cap;
   return unsigned(rounds > 0 ? (blocks + rounds - 1) / rounds : 1);
 }

@@ -4,9 +4,9 @@
 // The FP64 kernel issues 1957 FP64 instructions per iteration and is bound by that unit (0.92 of
 // its measured rate). Here the chain's kinematics, the Jacobian, the products with Jlog6 and the
 // normal matrix run on the integer pipes beside the ~370 FP64 instructions that remain.
-// Measured, 65536 9-DoF arms following targets, at most 100 iterations: 19.1 -> 10.1 ms; 16 of
+// Measured, 65536 9-DoF arms following targets, at most 100 iterations: 19.1 -> 8.5 ms; 16 of
 // them, 30 iterations: 2.3 -> 1.1 ms. Bound by the latency of its ~18000 instructions per
-// iteration (4.4 cycles each with under two warps per scheduler).
+// iteration (4.4 cycles each with under two warps per scheduler) and, with three, by their issue.
 //
 // Along the path to the link, u and p are each joint's world axis and position; with the link's
 // joint at (Ro, po) a revolute column in its frame is Ro^T (u x (po - p), u), so with
@@ -367,10 +367,19 @@ static __device__ __noinline__ void ik_env_fp64(const DModel* __restrict__ model
   ik_env<MAXJ>(model, a, e);
 }
 
-template <int MAXJ>
-__global__ void __launch_bounds__(32) bfp_ik_kernel(const DModel* __restrict__ model, const IkArgs a) {
+template <int MAXJ, int BLOCKS>
+__global__ void __launch_bounds__(32, BLOCKS) bfp_ik_kernel(const DModel* __restrict__ model, const IkArgs a) {
   for (int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; e < a.n; e += int64_t(gridDim.x) * blockDim.x)
     if (!bfp::ik_env<MAXJ>(model, a, e)) ik_env_fp64<MAXJ>(model, a, e);
+}
+
+// 168 registers hold all of an iteration, 12 warps per multiprocessor; batches beyond those take
+// the kernel of 144 registers and 14 warps, which costs a few spills and saves rounds (9-DoF
+// arms, 100 iterations: 65536 environments 10.1 -> 8.5 ms, but 30000: 4.8 -> 5.1 ms).
+template <int MAXJ>
+cudaError_t launch_bfp_ik(const DModel* dm, const IkArgs& a, cudaStream_t s) {
+  const bool all_resident = (a.n + 31) / 32 <= 12 * int64_t(multiprocessors());
+  return launch_ik_kernel(all_resident ? bfp_ik_kernel<MAXJ, 12> : bfp_ik_kernel<MAXJ, 14>, dm, a, s);
 }
 
 }  // namespace sgdyn
