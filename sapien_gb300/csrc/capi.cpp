@@ -761,7 +761,13 @@ int sgdyn_compute_forward_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(tau_bar, n, nv, layout);
-    if (Mo.bfp_ok()) {
+    // The integer sweep's cost grows with the tree's pairs and with n, the FP64 kernel's is flat up
+    // to a warp per scheduler: with long ancestor chains that one is the faster beyond it
+    // (18-DoF quadruped, 6.5 pairs per column, 16384 environments: 533 us against 556 in FP64,
+    // 24576: 800 against 651; 35-DoF humanoid, 32768: 2325 against 1654; 9-DoF arm, 4.9 pairs,
+    // 131072: 1371 against 1637).
+    const bool long_chains = Mo.btree().npairs > 6 * Mo.nv();
+    if (Mo.bfp_ok() && !(long_chains && n > 32 * int64_t(device_schedulers()))) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::aba_vjp, dm, bfp_tree(Mo), nullptr, &a,
                                             static_cast<cudaStream_t>(stream));
       if (e != cudaErrorNotSupported) return launch_status(e);

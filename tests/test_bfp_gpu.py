@@ -324,3 +324,23 @@ def test_inverse_kinematics_matches_fp64(name, n, steps):
         else:
             assert rel_per_env(a[keep], b[keep]) <= 1e-9
             assert (np.isfinite(a) == np.isfinite(b)).all()
+
+
+@pytest.mark.parametrize("name", ["quadruped", "arm9"])
+def test_forward_dynamics_vjp_on_both_sides_of_the_batch_size_rule(name):
+    """The largest batch that stays on one warp per scheduler, one environment more, and the same
+    environments in a small batch."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    edge = 32 * 4 * torch.cuda.get_device_properties(0).multi_processor_count
+    q, qd, _, tau = cuda(*robot.sample(edge + 1, seed=12))
+    w = torch.ones_like(qd)
+    small = AD.forward_dynamics_vjp(pm, q[-40:], qd[-40:], tau[-40:], w[-40:])
+    for n in (edge, edge + 1):
+        got = AD.forward_dynamics_vjp(pm, q[-n:], qd[-n:], tau[-n:], w[-n:])
+        for a, b in zip(got, small):
+            assert rel_per_env(a[-40:].cpu().numpy(), b.cpu().numpy()) <= 1e-9
