@@ -44,7 +44,7 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 KERNEL = "block floating point"
 KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39004134 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "3d0f82662d115f25457d8c0e34f2ba9d184bb41b9c92bbfe79a35e79109b18f4"
+KERNEL_SOURCE_SHA256 = "00c9f583aa58dc8328104091d4a7bb7756dbacc380823560773325efb456edae"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

@@ -315,6 +315,12 @@ int sgdyn_compute_forward_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
                                        const double* tau, const double* qdd_bar, double* q_bar, double* qd_bar,
                                        double* tau_bar, int layout, void* stream);
 
+/* Gradients with respect to q's tangent (rows [n][nv], as the products above give them) as
+ * gradients with respect to q's coordinates (rows [n][nq]): a free flyer's position gradient is
+ * R g_lin, its quaternion gradient has no component along the quaternion. Environment-major. */
+int sgdyn_tangent_to_coordinate_gradient(const sgdyn_model* m, int64_t n, const double* q, const double* g,
+                                         double* out, void* stream);
+
 /* Vector-Jacobian product of the link poses: pos_bar [n][nlinks*3] (adjoint of link
  * positions), rot_bar [n][nlinks*9] (adjoint of row-major link rotations) or NULL ->
  * q_bar [n][nv]. */

@@ -55,6 +55,7 @@ EXPORTED = (
     "sgdyn_compute_inverse_kinematics",
     "sgdyn_compute_inverse_dynamics_vjp",
     "sgdyn_compute_forward_dynamics_vjp",
+    "sgdyn_tangent_to_coordinate_gradient",
     "sgdyn_compute_forward_kinematics_vjp",
     "sgdyn_compute_rnea_derivatives",
     "sgdyn_compute_aba_derivatives",
@@ -142,6 +143,7 @@ def load():
                                                         i32]
     L.sgdyn_compute_inverse_dynamics_vjp.argtypes = [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, vp]
     L.sgdyn_compute_forward_dynamics_vjp.argtypes = [vp, i64, vp, vp, vp, vp, vp, vp, vp, i32, vp]
+    L.sgdyn_tangent_to_coordinate_gradient.argtypes = [vp, i64, vp, vp, vp, vp]
     L.sgdyn_compute_forward_kinematics_vjp.argtypes = [vp, i64, vp, vp, vp, vp, i32, vp]
     L.sgdyn_compute_rnea_derivatives.argtypes = [vp, i64, vp, vp, vp, vp, vp, vp, i32, vp]
     L.sgdyn_compute_aba_derivatives.argtypes = [vp, i64, vp, vp, vp, vp, vp, vp, i32, vp]

@@ -80,6 +80,18 @@ def tangent_to_coordinate_grad(model, q, g):
     return out
 
 
+def _coordinate_grad(model, q, g):
+    """tangent_to_coordinate_grad in one launch, for a backward pass that is not itself recorded."""
+    if model.nq_ext == model.nv or torch.is_grad_enabled():
+        return tangent_to_coordinate_grad(model, q, g)
+    q, g = _f64(q, model.nq_ext, "q"), g.contiguous()
+    out = torch.empty_like(q)
+    with torch.cuda.device(q.device):
+        N.check(N.load().sgdyn_tangent_to_coordinate_gradient(model._h, q.shape[0], _p(q), _p(g), _p(out),
+                                                              _stream(q.device)))
+    return out
+
+
 def coordinate_to_tangent_grad(model, q, gc):
     """[N, nq_ext] gradient with respect to q's coordinates -> [N, nv] tangent gradient (the
     transpose of the chart's derivative d q exp6(eps) / d eps at eps = 0)."""
@@ -198,7 +210,7 @@ class _InverseDynamics(torch.autograd.Function):
     def backward(ctx, tau_bar):
         q, qd, qdd = ctx.saved_tensors
         qb, qdb, qddb = inverse_dynamics_vjp(ctx.model, q, qd, qdd, tau_bar.contiguous())
-        return None, tangent_to_coordinate_grad(ctx.model, q, qb), qdb, qddb
+        return None, _coordinate_grad(ctx.model, q, qb), qdb, qddb
 
 
 class _ForwardDynamics(torch.autograd.Function):
@@ -212,7 +224,7 @@ class _ForwardDynamics(torch.autograd.Function):
     def backward(ctx, qdd_bar):
         q, qd, tau = ctx.saved_tensors
         qb, qdb, tb = forward_dynamics_vjp(ctx.model, q, qd, tau, qdd_bar.contiguous())
-        return None, tangent_to_coordinate_grad(ctx.model, q, qb), qdb, tb
+        return None, _coordinate_grad(ctx.model, q, qb), qdb, tb
 
 
 def _quat_to_R(qwxyz):
@@ -238,7 +250,7 @@ class _LinkPoses(torch.autograd.Function):
             pos_bar = torch.zeros(q.shape[0], ctx.model.nlinks, 3, dtype=q.dtype, device=q.device)
         qb = forward_kinematics_vjp(ctx.model, q, pos_bar.contiguous(),
                                     rot_bar.contiguous() if rot_bar is not None else None)
-        return None, tangent_to_coordinate_grad(ctx.model, q, qb)
+        return None, _coordinate_grad(ctx.model, q, qb)
 
 
 def inverse_dynamics(model, q, qd, qdd):
@@ -328,7 +340,7 @@ class _Rollout(torch.autograd.Function):
             qT_bar = _tangent_in_q_layout(m, coordinate_to_tangent_grad(m, qT, qT_bar))
         q0b, qd0b, taub = rollout_backward(m, qc, qdc, tau, ctx.dt, ctx.K, qT_bar, qdT_bar)
         if m.nq_ext != m.nv:
-            q0b = tangent_to_coordinate_grad(m, q0, _tangent_from_q_layout(m, q0b))
+            q0b = _coordinate_grad(m, q0, _tangent_from_q_layout(m, q0b))
         return None, q0b, qd0b, taub, None, None
 
 

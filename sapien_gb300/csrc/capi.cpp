@@ -801,6 +801,22 @@ int sgdyn_compute_forward_kinematics_vjp(const sgdyn_model* m, int64_t n, const 
   });
 }
 
+int sgdyn_tangent_to_coordinate_gradient(const sgdyn_model* m, int64_t n, const double* q, const double* g, double* out,
+                                         void* stream) {
+  SG_TRACE("sgdyn_tangent_to_coordinate_gradient");
+  return guarded([&] {
+    if (int rc = check_diff_model(m)) return rc;
+    if (int rc = common_checks(n, SGDYN_ENV_MAJOR)) return rc;
+    if (n == 0) return SGDYN_OK;
+    if (int rc = check_ptrs({{q, "q"}, {g, "g"}, {out, "out"}})) return rc;
+    int err = 0;
+    const DModel* dm = m->impl->device_table(&err);
+    if (!dm) return fail(SGDYN_ERR_CUDA, "model upload failed");
+    return launch_status(launch_tangent_to_coordinate(dm, m->impl->njoints(), n, q, g, out,
+                                                      static_cast<cudaStream_t>(stream)));
+  });
+}
+
 static int derivatives(bool aba, const sgdyn_model* m, int64_t n, const double* q, const double* qd, const double* x,
                        double* d_q, double* d_qd, double* d_x, int layout, void* stream) {
   return guarded([&] {

@@ -146,6 +146,9 @@ cudaError_t launch_bfp_passive(const DModel* dm, const BfpTree& t, const Passive
 enum class BfpDiff { rollout, replay, reverse, rnea_vjp, aba_vjp };
 cudaError_t launch_bfp_diff(BfpDiff what, const DModel* dm, const BfpTree& t, const RolloutArgs* r, const VjpArgs* v,
                             cudaStream_t s);
+// Env-major rows of tangent gradients g at q to coordinate gradients.
+cudaError_t launch_tangent_to_coordinate(const DModel* dm, int nj, int64_t n, const double* q, const double* g,
+                                         double* out, cudaStream_t s);
 // Doubles per environment and step of the replay's records.
 int64_t bfp_record_doubles(const BfpTree& t);
 // Forward dynamics alone with three lanes per environment (team3.cuh; one-DoF joints and a

@@ -344,3 +344,23 @@ def test_forward_dynamics_vjp_on_both_sides_of_the_batch_size_rule(name):
         got = AD.forward_dynamics_vjp(pm, q[-n:], qd[-n:], tau[-n:], w[-n:])
         for a, b in zip(got, small):
             assert rel_per_env(a[-40:].cpu().numpy(), b.cpu().numpy()) <= 1e-9
+
+
+@pytest.mark.parametrize("name,n", [("quadruped", 1), ("quadruped", 37), ("mixed", 5), ("humanoid", 300)])
+def test_coordinate_gradients_in_one_launch(name, n):
+    """The launch behind a backward pass against the tensor operations of the public function: a
+    few FP64 products and sums of unit size apart."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    (q,) = cuda(robot.sample(n, seed=1)[0])
+    g = torch.randn(n, pm.nv, generator=torch.Generator().manual_seed(0), dtype=torch.float64).cuda()
+    pm._prepare(q.device)
+    want = AD.tangent_to_coordinate_grad(pm, q, g)
+    with torch.no_grad():
+        got = AD._coordinate_grad(pm, q, g)
+    assert got.shape == want.shape
+    assert float((got - want).abs().max()) <= 32 * 2.0**-53 * float(g.abs().max()) * 4
