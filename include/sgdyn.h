@@ -172,16 +172,22 @@ int sgdyn_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const 
  * environments (CRBA + RNEA + ABA on `stream`, FK + Jacobian on an internal second stream of
  * the device, ordered after the work already on `stream` and before what follows there; the
  * FK + Jacobian warps repeat the joint placements but fill FP64 schedulers the others leave
- * idle), 2 automatic (the default: two launches while the batch gives fewer than two warps
- * per FP64 scheduler and `stream` is not being captured), -1 only reads the mode. Results
- * agree to rounding. (Addition.) */
+ * idle), 2 automatic (the default), -1 only reads the mode. Results agree to rounding.
+ * Automatic, with lanes per environment and forward-dynamics method automatic too: one launch of
+ * the block sweep for any set of ops (block floating point, a block of threads per group of
+ * environments), for every model with constants that are 0 or within 2^+-100 and a tree that
+ * fits a block's shared memory. Other models, and any other value of these settings: the FP64
+ * kernels, as two launches while the batch gives fewer than two warps per FP64 scheduler and
+ * `stream` is not being captured. Modes 0 and 1 also keep mixed batches and inverse kinematics
+ * in FP64. (Addition.) */
 int sgdyn_step_split(int mode, int* mode_out);
 
 /* Lanes per environment for the single-model fused sweep and single-op entry points
  * (addition): 0 = automatic (default), 1, 2, 4 or 8. With L > 1 a team of L lanes shares an
  * environment: the joints near the root run on every lane and the subtrees off them on one
  * lane each, which shortens a wide tree's sequential sweep; worth it when the batch leaves
- * the GPU's FP64 schedulers idle (automatic: only then, and only if the tree splits). */
+ * the GPU's FP64 schedulers idle (automatic: the block sweep, see sgdyn_step_split; for models
+ * it cannot hold, teams only then, and only if the tree splits). */
 int sgdyn_model_set_lanes(sgdyn_model* m, int lanes);
 /* The team table the kernels use for `lanes` lanes per environment (ints: L, trunk count,
  * longest lane, attach count, trunk joints, per-lane joints padded with 0, attach joints,
@@ -208,7 +214,8 @@ int sgdyn_jit_config(int enable, int64_t min_n, int* enabled, int64_t* min_n_out
 /* Size limit of run-time specialisation (joints incl. the universe; < 0 leaves it). */
 int sgdyn_jit_max_joints(int max_joints, int* max_joints_out);
 /* How the run-time-specialised sweep computes forward dynamics (addition): 0 automatic (the
- * default: the route with fewer FP64 operations for the model and op set), 1 the
+ * default: the block sweep, see sgdyn_step_split; in FP64 the route with fewer operations for the
+ * model and op set), 1 the
  * articulated-body passes (ABA), 2 from the mass matrix (CRBA, the bias forces by RNEA at
  * zero acceleration, M = L^T D L with the tree's sparsity, qdd = M^-1 (tau - b); inverse
  * dynamics in the same sweep then reads tau = b + M qdd); -1 only reads the setting.
@@ -260,7 +267,7 @@ int sgdyn_host_compute_inverse_kinematics(const sgdyn_model* m, int64_t n, int l
                                           int layout, int nthreads);
 
 /* ---- heterogeneous batches (addition: the reference evaluates one robot per call) ------
- * Robots of different size and topology in one persistent launch. A batch is planned once
+ * Robots of different size and topology stepped together. A batch is planned once
  * (tables packed, environments grouped per model into tiles of up to 32, tiles ordered by
  * descending velocity dimension) and stepped many times; a step allocates nothing, so it
  * can be recorded into a CUDA graph. Arrays are row-major and padded to the batch maxima:
@@ -282,6 +289,8 @@ int sgdyn_batch_set_launch(sgdyn_batch* b, int ctas_per_sm, int warps_per_cta, i
  * subtrees hanging off them on one lane each, so a wide tree's sequential sweep gets
  * shorter at the price of more lanes. Chosen by sapien_gb300.autotune. Re-plans the batch
  * (allocates): not while a stream of the batch's device is being captured. */
+/* (Launch shapes and lanes are those of the FP64 kernels: a batch whose models all fit the block
+ * sweep takes one launch of it per model, see sgdyn_step_split.) */
 int sgdyn_batch_set_lanes(sgdyn_batch* b, const int* lanes_per_model);
 int sgdyn_batch_step(sgdyn_batch* b, int ops, const double* q, const double* qd, const double* qdd, const double* tau,
                      double* link_poses, double* J, double* M, double* tau_out, double* qdd_out, void* stream);
@@ -355,7 +364,8 @@ int sgdyn_rollout_forward(const sgdyn_model* m, int64_t n, int T, double dt, con
 /* Lanes per environment of the ABA-based sweeps: sgdyn_rollout_forward, the reverse sweep
  * of sgdyn_rollout_backward / _noalloc, and forward dynamics requested alone
  * (sgdyn_compute_forward_dynamics, sgdyn_step with only SGDYN_OP_FORWARD_DYNAMICS)
- * (addition): 0 automatic (the default:
+ * (addition): 0 automatic (the default: the
+ * block sweeps, see sgdyn_step_split; for models they cannot hold
  * three lanes while one warp per ten environments leaves no FP64 scheduler with two warps),
  * 1, or 3 (one lane per Cartesian axis of every spatial quantity, warp shuffles between
  * them, so each lane issues about half the FP64 instructions of one lane per environment;

@@ -1,4 +1,4 @@
-"""Heterogeneous batches: several robot models stepped together in one persistent launch.
+"""Heterogeneous batches: several robot models stepped together.
 
     batch = HeteroBatch([arm, quadruped, humanoid], model_of_env)   # plan once
     q = batch.pad_q([q_arm, q_quad, q_hum])                          # padded [N, max_nq]
@@ -6,11 +6,13 @@
     graph = batch.capture(q, qd, qdd, tau, steps=10)                 # CUDA graph of 10 steps
     graph.replay()
 
-Environments are grouped per model into warps (tiles of 32 / L environments for a model
-run with L lanes per environment) and the tiles are ordered by descending velocity
-dimension; a persistent grid pulls tiles from an atomic counter (see csrc/hetero.cu). The
-launch shape (persistent CTAs per SM, warps per CTA, tile order) and the lanes per
-environment of each model are chosen by ``sapien_gb300.autotune.tune_batch``.
+A step is one launch of the block sweep per model on its rows of the padded arrays, side by
+side on streams of the batch (see csrc/hetero.cu). For models out of that sweep's range, or
+with FP64 forced, environments are grouped per model into warps (tiles of 32 / L environments
+for a model run with L lanes per environment), ordered by descending velocity dimension, and a
+persistent grid pulls tiles from an atomic counter; its launch shape (persistent CTAs per SM,
+warps per CTA, tile order) and the lanes per environment of each model are chosen by
+``sapien_gb300.autotune.tune_batch``.
 """
 from __future__ import annotations
 
@@ -121,7 +123,8 @@ class HeteroBatch:
         return out
 
     def step(self, q, qd=None, qdd=None, tau=None, ops=OPS_DYNAMICS, out=None):
-        """One persistent launch over all environments; returns the (padded) outputs."""
+        """One step of all environments, a launch of the block sweep per model side by side (or one
+        persistent FP64 launch, see sgdyn_step_split); returns the (padded) outputs."""
         out = out if out is not None else self.alloc_outputs(ops)
         with torch.cuda.device(self.device):
             N.check(N.load().sgdyn_batch_step(
@@ -138,7 +141,7 @@ class HeteroBatch:
                                                    ctypes.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)))
 
     def rollout_step(self, q, qd, tau, dt, out):
-        """One rollout step in place and in one launch: qdd = ABA(q, qd, tau) into
+        """One rollout step in place, the update fused into the sweep: qdd = ABA(q, qd, tau) into
         out["qacc"], then the semi-implicit Euler update of `integrate`, each environment
         right after its own sweep (bitwise the same as `step` + `integrate`)."""
         with torch.cuda.device(self.device):
