@@ -44,7 +44,7 @@ WORKLOAD = ("arm9: 9-DoF tree (7 revolute + 2 prismatic fingers), N=16384 envs p
 KERNEL = "block floating point"
 KERNEL_COUNTERS = {"fp64_inst_per_env": 2785280 / 16384, "warp_inst_per_env": 39004134 / 16384,
                    "dram_bytes_per_env": 4.87e6 / 16384}
-KERNEL_SOURCE_SHA256 = "00c9f583aa58dc8328104091d4a7bb7756dbacc380823560773325efb456edae"
+KERNEL_SOURCE_SHA256 = "e12448bbfb7f4a46fbb7a1ef099242137e3eb26083234ee7b5f50e2343bdfbb7"
 KERNEL_HEADERS = ("device_model.h", "kernels.h", "spatial.cuh", "bfp.cuh", "bfp_block.cuh")
 
 

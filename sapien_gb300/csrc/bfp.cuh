@@ -92,7 +92,6 @@ SG_HD unsigned abs_hi(i64 m) {
   return unsigned(h < 0 ? -h : h);
 }
 SG_HD int imax(int a, int b) { return a > b ? a : b; }
-SG_HD int imin(int a, int b) { return a < b ? a : b; }
 
 // Dot products of one to three pairs: cross terms first, their high word carried into the sum of
 // the high terms. The result is in units of 2^64 times the operands' units.
@@ -328,17 +327,12 @@ struct Q3 {
 SG_HD Q3 split4(i64 x, i64 y, i64 z) { return Q3{split4(x), split4(y), split4(z)}; }
 SG_HD i64 dot60(Q3 a, Q3 b) { return mul60(a.x, b.x, a.y, b.y, a.z, b.z); }
 SG_HD H3 row(const Rot& R, int i) { return H3{split(R.a[3 * i]), split(R.a[3 * i + 1]), split(R.a[3 * i + 2])}; }
-SG_HD H3 col(const Rot& R, int j) { return H3{split(R.a[j]), split(R.a[3 + j]), split(R.a[6 + j])}; }
 SG_HD Q3 row4(const Rot& R, int i) { return split4(R.a[3 * i], R.a[3 * i + 1], R.a[3 * i + 2]); }
 SG_HD Q3 col4(const Rot& R, int j) { return split4(R.a[j], R.a[3 + j], R.a[6 + j]); }
 SG_HD Vec col_vec(const Rot& R, int j) { return Vec{R.a[j], R.a[3 + j], R.a[6 + j], -60}; }
 SG_HD Vec mul(const Rot& R, Vec v) {
   const H3 h = split(v);
   return Vec{dot(row(R, 0), h), dot(row(R, 1), h), dot(row(R, 2), h), v.e + 4};
-}
-SG_HD Vec mulT(const Rot& R, Vec v) {
-  const H3 h = split(v);
-  return Vec{dot(col(R, 0), h), dot(col(R, 1), h), dot(col(R, 2), h), v.e + 4};
 }
 SG_HD Rot mul(const Rot& A, const Rot& B) {
   Rot C;
@@ -406,13 +400,10 @@ SG_HD void rot_quat(const Rot& R, double* q) {
 }
 
 // ---- spatial vectors and inertias ------------------------------------------------------
-SG_HD Tw tw0() { return Tw{vec0(), vec0()}; }
 SG_HD Tw norm(Tw a) { return Tw{norm(a.v), norm(a.w)}; }
 SG_HD Tw add(Tw a, Tw b) { return Tw{add(a.v, b.v), add(a.w, b.w)}; }
 SG_HD Tw neg(Tw a) { return Tw{neg(a.v), neg(a.w)}; }
 SG_HD Tw mul(Sc s, Tw a) { return Tw{mul(s, a.v), mul(s, a.w)}; }
-// s x + y
-SG_HD Tw axpy(Sc s, Tw x, Tw y) { return add(mul(s, x), y); }
 SG_HD Sc dot(Tw a, Tw b) { return add(dot(a.v, b.v), dot(a.w, b.w)); }
 // motion x motion and motion x* force
 SG_HD Tw crossm(Tw a, Tw b) {
