@@ -12,8 +12,14 @@
 // them, so a 3 x 3 product costs ~450 cycles a warp against ~2150 in FP64 (probe, two warps
 // per scheduler and more). Up to three products fit the accumulators.
 //
-// Precision: a mantissa keeps 60 bits below the largest component of its vector and a product
-// or dot product is off by about 2^-57 of |a| |b|, against 2^-53 for one rounded FP64 operation. Inputs are converted exactly, results are rounded to nearest once.
+// Precision: all bounds are relative to the largest component of a vector, matrix or rotation. A
+// mantissa keeps 60 bits below it and a product or dot product is off by about 2^-57 of |a| |b|,
+// against 2^-53 for one rounded FP64 operation. A number on its own converts exactly; beside a
+// larger one it is cut off 60 bits below that, as are the terms of a sum, where FP64 keeps 53
+// bits of each: a component more than 2^7 below the largest holds less here than there. Rotations
+// and sines are in steps of 2^-60 at any size. So callers keep configurations with small angles
+// (bfp_small) away from these routines, and results that are small against their terms. Results
+// are rounded to nearest once, on their way out.
 //
 // Range: exponents are 32-bit integers, so nothing overflows between inputs and outputs. Callers
 // keep inputs that are not finite or beyond 2^+-200 away from these routines (bfp_fits).
@@ -163,6 +169,15 @@ SG_HD bool bfp_fits(double x) {
   const unsigned E = unsigned(b >> 52) & 0x7ffu;
   return (b << 1) == 0 || (E - 823u) < 400u;
 }
+// Not 0, but below 2^-kSmall. The sine of an angle at that edge is held to 2^-44 of itself, a
+// product with it to 2^-41. An environment with such an angle may have to go through FP64, which
+// takes as long again: with kSmall = 12 a fifth longer for 16384 9-DoF arms with random angles,
+// with 16 no longer (three batches in four have no angle below 2^-14, eleven in twelve below 2^-16).
+constexpr int kSmall = 16;
+SG_HD bool bfp_small(double x) {
+  const u64 b = dbits(x) << 1;
+  return b != 0 && unsigned(b >> 53) < unsigned(1023 - kSmall);
+}
 // x = m 2^e with 2^60 <= |m| < 2^61 (0: m = 0); exact
 SG_HD Sc from_double(double x) {
   const u64 b = dbits(x);
@@ -241,9 +256,10 @@ SG_HD i64 rsqrt60(i64 v) {
   return shl(i64(y), 32) + shl(wide(ch.h, y, 0), 4) + (wide(ch.l, y, 0) >> 28);
 }
 
-// Sine and cosine of x as mantissas of exponent -60: x in fixed point 2^-58, reduced by
+// Sine and cosine of x as mantissas of exponent -60: x in fixed point 2^-60, reduced by
 // multiples of pi/2 (constant in two parts), Taylor polynomials on [-pi/4, pi/4]. The terms
 // that weigh less than 2^-28 are summed in 32-bit products. |x| >= 24 goes through the library.
+// Off by 2^-56; a sine of a small angle by 2^-60.
 SG_HD void sincos60(double x, i64* s, i64* c) {
   if (!(x > -24.0 && x < 24.0)) {
     double ds, dc;
@@ -254,11 +270,12 @@ SG_HD void sincos60(double x, i64* s, i64* c) {
   }
   const Sc xs = from_double(x);
   const int sh = xs.e + 58;  // at most 2
-  const i64 q = sh > 0 ? shl(xs.m, sh) : shr(xs.m, -sh);
-  const int n = int((wide(hi32(q), 1367130551, 0) + (1LL << 56)) >> 57);  // x 2/pi rounded (2/pi in 2^-31)
-  // x - n pi/2 (pi/2 = 452751216129820178 - 1507445996 2^-32 in units of 2^-58)
-  i64 r = q - i64(n) * 452751216129820178LL + (wide(n, 1507445996, 0) >> 32);
-  r = shl(r, 2);
+  const i64 h = sh > 0 ? shl(xs.m, sh) : shr(xs.m, -sh);
+  const int n = int((wide(hi32(h), 1367130551, 0) + (1LL << 56)) >> 57);  // x 2/pi rounded (2/pi in 2^-31)
+  // x in units of 2^-60 rounded to nearest, and x - n pi/2 (pi/2 = 1811004864519280711 -
+  // 1734816687 2^-32 in these units); what goes beyond 64 bits on the way cancels
+  const i64 q = sh >= -2 ? shl(xs.m, sh + 2) : shr(shr(xs.m, -sh - 3) + 1, 1);
+  const i64 r = i64(u64(q) - u64(n) * 1811004864519280711ULL) + (wide(n, 1734816687, 0) >> 32);
   const i64 z = mul60(r, r);
   const int zh = int(z >> 29);
   auto m31 = [](int a, int b) { return int(wide(a, b, 0) >> 31); };
@@ -281,7 +298,9 @@ SG_HD void sincos60(double x, i64* s, i64* c) {
   C = step(C) - 1601279867509510LL;    // 1 / 6!
   C = step(C) + 48038396025285291LL;   // 1 / 4!
   C = step(C) - 576460752303423488LL;  // 1 / 2!
-  const i64 sn = r + mul60(r, step(S));
+  // r S with the low product, which weighs up to 2^-58: a small sine is kept to 2^-59
+  const Half4 rs = split4(r), ss = split4(step(S));
+  const i64 sn = r + wide(rs.h4, ss.h4, (cross_terms(rs, ss, kRound4) + (wide(rs.l, ss.l, 0) >> 32)) >> 28);
   const i64 cs = kOne + step(C);
   const i64 a = (n & 1) ? cs : sn, b = (n & 1) ? sn : cs;
   *s = (n & 2) ? -a : a;

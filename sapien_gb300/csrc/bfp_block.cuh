@@ -36,7 +36,7 @@ namespace sgdyn {
 namespace bfp {
 
 // Shared-memory items per environment: 64-bit words and exponents of a model's state.
-//   in: q, qd, qdd, tau
+//   in: q, qd, qdd, tau; for adjoint sweeps one more per column, for adjoints that go in
 //   A: per joint, rotation (9) + position (3), later acceleration (6) + force (6); then the
 //      scaled factor's entries
 //   Y: per joint, first the joint's own rotation (9), then mass, first moment, inertia (10);
@@ -44,7 +44,7 @@ namespace bfp {
 //   S, V: per column 6 (V: per joint velocity, then column forces); then L in FP64
 //   b: per column, right-hand side and solution
 //   u: for adjoint sweeps (bfp_diff.cuh), per joint 6; there Y has 12 per joint for two wrenches
-// After them the tree's ints (BTree), once per block.
+// After them the tree's ints (BTree), once per block, and the environments' notes, twice.
 struct BlkLayout {
   int in, A, Y, S, V, b, u, words;    // word items
   int xA, xY, xS, xV, xs, xu, ints;   // exponent items
@@ -53,7 +53,7 @@ SG_HD BlkLayout blk_layout(int nj, int nv, int nq, int npairs, bool adjoint = fa
   const int m = nj - 1;
   BlkLayout L;
   L.in = 0;
-  L.A = nq + 3 * nv;
+  L.A = nq + (adjoint ? 4 : 3) * nv;
   L.Y = L.A + imax(12 * m, npairs);
   L.S = L.Y + imax((adjoint ? 12 : 10) * m, npairs);
   L.V = L.S + 6 * nv;
@@ -66,12 +66,28 @@ SG_HD BlkLayout blk_layout(int nj, int nv, int nq, int npairs, bool adjoint = fa
   L.xV = L.xS + 2 * nv;
   L.xs = L.xV + 2 * nv;  // scale and pivot shift of each column
   L.xu = L.xs + 2 * nv;  // u (2 per joint), and Y as two wrenches (4 per joint)
-  L.ints = L.xu + (adjoint ? 6 * m : 0) + 1;  // and whether the environment needs the FP64 sweep
+  L.ints = L.xu + (adjoint ? 6 * m : 0);
   return L;
 }
+// What a sweep notes of an environment on its way, for the question whether its results have to
+// come from the FP64 algebra (Blk::refused). All but NOTE_REFUSED are the largest binary exponent
+// of something, kNoNote where there was nothing.
+enum Note : int {
+  NOTE_REFUSED,  // an input, a pivot or an adjoint out of range
+  NOTE_SCALE,    // products that the bodies' forces are summed from
+  NOTE_BIAS,     // generalised bias forces (inverse dynamics)
+  NOTE_DRIVE,    // applied generalised forces
+  NOTE_TORQUE,   // inverse dynamics out of M qdd + bias
+  NOTE_GSCALE,   // products that the gradient with respect to q is summed from
+  NOTE_GRAD,     // that gradient
+  kNotes
+};
+constexpr int kNoNote = -4000;
+// binary digits of a row that may be lost, see Blk::refused: of forces, of gradients, of float32
+constexpr int kLost = 7, kLostGrad = 12, kLostFloat = 24;
 constexpr int kBlkMaxThreads = 640, kBlkDiffThreads = 512;
 SG_HD size_t blk_bytes(const BlkLayout& L, int tree_ints, int E) {
-  return size_t(E) * (8 * size_t(L.words) + 4 * size_t(L.ints)) + 4 * size_t(tree_ints);
+  return size_t(E) * (8 * size_t(L.words) + 4 * size_t(L.ints) + 2 * 4 * size_t(kNotes)) + 4 * size_t(tree_ints);
 }
 
 // World motion subspace column k of joint J at pose (Ro, po).
@@ -88,9 +104,8 @@ SG_HD Tw joint_S(const DJoint& J, const BJoint& B, const Rot& Ro, Vec po, int k)
 #ifdef __CUDACC__
 // The two algebras a block sweep runs in. BfpAlg: block floating point. FpAlg: plain FP64 on
 // the same phases and shared-memory items (mantissa words hold doubles), for environments that
-// BfpAlg turns away: inputs that are not finite or beyond 2^+-200, quaternions off unit
-// length, a mass matrix that is not safely positive definite. Calls on their types are found
-// in the types' namespaces (bfp.cuh; below for the FP64 ones).
+// BfpAlg turns away (Blk::refused). Calls on their types are found in the types' namespaces
+// (bfp.cuh; below for the FP64 ones).
 struct BfpAlg {
   static constexpr bool kFixed = true;
   typedef bfp::Sc Sc;
@@ -198,7 +213,10 @@ __device__ __forceinline__ V3 col_vec(const M3& R, int j) { return mk(R.a[j], R.
 
 namespace bfp {
 
-template <class A, int E>
+// The block's state as algebra A sees it, E environments side by side (0: as many as a pass
+// needs). EI: environments of the block, the stride of the inputs and notes, which keep their
+// place when the algebra changes.
+template <class A, int E, int EI = E>
 struct Blk {
   typedef typename A::Vec Vec;
   typedef typename A::Rot Rot;
@@ -210,17 +228,25 @@ struct Blk {
   const int* pair_of;  // in global memory
   int nj, nv, nq, levels, npairs, col_levels;
   BlkLayout L;
-  i64* w;
-  int* x;
+  i64 *w, *win;
+  int *x, *note_base;
   // the tree's arrays, in shared memory
   const int *parent, *end, *level, *order, *level_start, *col_joint, *col_dof, *depth, *ext, *row_start, *col_order,
       *col_level_start, *pair_row, *pair_col;
-  int lane, slot, slots;  // this thread's environment in the block, its slot, slots per environment
+  int width;               // environments side by side, where E is 0
+  int lane, slot, slots;   // this thread's place among them, its slot, slots per environment
+  int el;                  // this thread's environment in the block
+  int count;               // environments whose results are written (the first lanes)
+  unsigned mask;           // which ones they are, where E is 0
+  bool valid;              // whether this thread's is one of them
+  int set;                 // which of the two sets of notes is in use
   int col;       // the slot's column (-1: none)
   int j, p, lv;  // the slot's joint (0: none), its parent and level
   double g[3];   // gravity
 
-  __device__ __forceinline__ void init(const DModel* model, long long* smem, bool adjoint = false) {
+  __device__ __forceinline__ int stride() const { return E ? E : width; }
+  // Copies the tree too, unless `again`: another pass over a block that is set up.
+  __device__ __forceinline__ void setup(const DModel* model, long long* smem, bool adjoint, bool again) {
     m = model;
     const BTree t = *model_btree(model);
     const int* ti = reinterpret_cast<const int*>(model_btree(model) + 1);
@@ -234,11 +260,15 @@ struct Blk {
     col_levels = t.col_levels;
     pair_of = ti + t.pair_of;
     L = blk_layout(nj, nv, nq, npairs, adjoint);
-    w = smem;
-    x = reinterpret_cast<int*>(smem + L.words * E);
-    int* s = x + L.ints * E;
+    win = smem;
+    w = smem + L.A * (EI - stride());  // the items after the inputs begin where the inputs end
+    x = reinterpret_cast<int*>(smem + L.words * EI);
+    int* s = x + L.ints * EI;
+    if (!again) {
 #pragma unroll 1
-    for (int k = threadIdx.x; k < t.nints; k += blockDim.x) s[k] = ti[k];
+      for (int k = threadIdx.x; k < t.nints; k += blockDim.x) s[k] = ti[k];
+    }
+    note_base = s + t.nints;
     parent = s + t.parent;
     end = s + t.end;
     level = s + t.level;
@@ -253,19 +283,49 @@ struct Blk {
     col_level_start = s + t.col_level_start;
     pair_row = s + t.pair_row;
     pair_col = s + t.pair_col;
-    lane = threadIdx.x % E;
-    slot = threadIdx.x / E;
-    slots = blockDim.x / E;
+    lane = int(threadIdx.x % unsigned(stride()));
+    slot = int(threadIdx.x / unsigned(stride()));
+    slots = int(blockDim.x / unsigned(stride()));
     col = slot < nv ? slot : -1;
     j = slot < nj - 1 ? slot + 1 : 0;
     for (int k = 0; k < 3; k++) g[k] = model->gravity[k];
     p = ti[t.parent + j];
     lv = ti[t.level + j];
   }
-  __device__ __forceinline__ i64& W(int item) const { return w[item * E + lane]; }
-  __device__ __forceinline__ int& X(int item) const { return x[item * E + lane]; }
-  __device__ __forceinline__ double D(int item) const { return __longlong_as_double(w[item * E + lane]); }
-  __device__ __forceinline__ void setD(int item, double v) const { w[item * E + lane] = __double_as_longlong(v); }
+  // The first `envs` of the block's environments.
+  __device__ __forceinline__ void init(const DModel* model, long long* smem, int envs, bool adjoint = false) {
+    setup(model, smem, adjoint, false);
+    el = lane;
+    count = envs;
+    valid = lane < envs;
+    set = 0;
+  }
+  // Those in `which` (E = 0), packed side by side so that a few of them take a few warps' issue.
+  // Lanes beyond them repeat the last one and share its inputs: only valid ones may change these.
+  __device__ __forceinline__ void init_some(const DModel* model, long long* smem, unsigned which, int note_set,
+                                            bool adjoint = false) {
+    mask = which;
+    count = __popc(which);
+    width = count <= 1 ? 1 : 1 << (32 - __clz(count - 1));
+    setup(model, smem, adjoint, true);
+    valid = lane < count;
+    el = env_at(min(lane, count - 1));
+    set = note_set;
+  }
+  // the environment in the block of a lane below `count`
+  __device__ __forceinline__ int env_at(int l) const {
+    if constexpr (E) return l;
+    unsigned r = mask;
+    for (int k = 0; k < l; k++) r &= r - 1;
+    return __ffs(int(r)) - 1;
+  }
+  __device__ __forceinline__ i64& W(int item) const { return w[item * stride() + lane]; }
+  __device__ __forceinline__ int& X(int item) const { return x[item * stride() + lane]; }
+  __device__ __forceinline__ double D(int item) const { return __longlong_as_double(w[item * stride() + lane]); }
+  __device__ __forceinline__ double D(int item, int l) const { return __longlong_as_double(w[item * stride() + l]); }
+  __device__ __forceinline__ void setD(int item, double v) const { w[item * stride() + lane] = __double_as_longlong(v); }
+  __device__ __forceinline__ double in(int c) const { return __longlong_as_double(win[c * EI + el]); }
+  __device__ __forceinline__ void set_in(int c, double v) const { win[c * EI + el] = __double_as_longlong(v); }
   __device__ __forceinline__ Vec vec(int item, int xi) const {
     if constexpr (A::kFixed) return Vec{W(item), W(item + 1), W(item + 2), X(xi)};
     else return Vec{D(item), D(item + 1), D(item + 2)};
@@ -349,12 +409,49 @@ struct Blk {
   __device__ __forceinline__ Tw frc(int j) const { return tw(iA(j) + 6, xA(j) + 2); }
   __device__ __forceinline__ void put_frc(int j, Tw v) const { put(iA(j) + 6, xA(j) + 2, v); }
 
-  __device__ __forceinline__ void refuse() const { X(L.ints - 1) = 1; }
-  __device__ __forceinline__ double q(int c) const { return D(L.in + c); }
-  __device__ __forceinline__ double qd(int c) const { return D(L.in + nq + c); }
-  __device__ __forceinline__ double qdd(int c) const { return D(L.in + nq + nv + c); }
-  __device__ __forceinline__ double tau(int c) const { return D(L.in + nq + 2 * nv + c); }
+  __device__ __forceinline__ double q(int c) const { return in(c); }
+  __device__ __forceinline__ double qd(int c) const { return in(nq + c); }
+  __device__ __forceinline__ double qdd(int c) const { return in(nq + nv + c); }
+  __device__ __forceinline__ double tau(int c) const { return in(nq + 2 * nv + c); }
+
+  // Notes; the FP64 algebra keeps none.
+  __device__ __forceinline__ int& note_at(int s, int note) const { return note_base[(s * kNotes + note) * EI + el]; }
+  __device__ __forceinline__ void clear_notes(int s) const {
+    if (slot == 0) {
+      for (int k = 0; k < kNotes; k++) note_at(s, k) = k == NOTE_REFUSED ? 0 : kNoNote;
+    }
+  }
+  __device__ __forceinline__ void refuse() const {
+    if constexpr (A::kFixed) note_at(set, NOTE_REFUSED) = 1;
+  }
+  __device__ __forceinline__ void note(Note k, int exponent) const {
+    if constexpr (A::kFixed) atomicMax(&note_at(set, k), exponent);
+  }
+  __device__ __forceinline__ void note(Note k, double v) const {
+    note(k, (__double2hiint(v) >> 20 & 0x7ff) - 1023);
+  }
+  // Whether the environment has to come from the FP64 algebra: refused on its way; or bits were
+  // lost that FP64 may keep. A vector here holds all its components to 2^-57 of the largest,
+  // FP64 each to 2^-53 of itself, so a whole row of results that is the small remainder of large
+  // terms (gravity torques next to an equilibrium, slow motion across gravity) may be exact in
+  // FP64 only. lost = kLost: where a row is below 2^-7 of its terms, so that an error of 2^-57 of
+  // the terms is at most 2^-50 of the row. Gradients (kLostGrad) are often that much smaller
+  // than their terms about the world's origin, where FP64 loses as much: 2^-45 of the row, about
+  // FP64's own error for 9-DoF arms. Results that cancel against applied forces cancel in FP64 too.
+  __device__ __forceinline__ bool refused(int lost = kLost) const {
+    if constexpr (!A::kFixed) return false;
+    const int scale = note_at(set, NOTE_SCALE), least = scale - lost, bias = note_at(set, NOTE_BIAS);
+    const int drive = note_at(set, NOTE_DRIVE), torque = note_at(set, NOTE_TORQUE);
+    const bool driven = (drive != kNoNote || torque != kNoNote) && (drive == kNoNote || drive >= least) &&
+                        (torque == kNoNote || torque >= least);
+    const int gscale = note_at(set, NOTE_GSCALE);
+    return note_at(set, NOTE_REFUSED) != 0 || (scale > kTiny && bias != kNoNote && bias < least && !driven) ||
+           (gscale > kTiny && note_at(set, NOTE_GRAD) < gscale - kLostGrad);
+  }
+  static constexpr int kTiny = -600;  // below: the terms are 0
 };
+
+__device__ __forceinline__ bool turns(const DJoint& J) { return J.kind == JK_REVOLUTE || J.kind == JK_CONTINUOUS; }
 
 // The joint's rotation after its placement, R_placement M_J(q).
 template <class A, class Q>
@@ -366,9 +463,42 @@ __device__ __forceinline__ typename A::Rot joint_rotation(const DJoint& J, const
   return rot_id ? r : mul(A::placement(J, B), r);
 }
 
-// World rotations and positions of all joints into A.
-template <class A, int E>
-__device__ __forceinline__ void blk_poses(const Blk<A, E>& b) {
+// Refuses the environment for its configuration, given its world rotations: a free flyer's
+// quaternion off unit length, and small angles that FP64 would hold to more bits. Rotations are in
+// steps of 2^-60 here, so what is proportional to a small angle keeps fewer bits of it. FP64 keeps
+// them only where the angle's sine is not added to something larger: where the rotation maps an
+// axis of the joint's frame on one of the world's, or nearly (an entry above kAligned, so two of
+// its row and column below 2^-10), as with joint axes along the frames' axes or on a root joint.
+// (Of a quaternion: where two components are small.)
+constexpr i64 kAligned = kOne - (kOne >> 21);
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_check_configuration(const Blk<A, E, EI>& b) {
+  if constexpr (!A::kFixed) return;
+  if (!b.j) return;
+  const DJoint& J = b.J[b.j];
+  if (J.kind == JK_FREEFLYER) {
+    float n2 = 0;
+    int small = 0, zeros = 0;
+    for (int k = 3; k < 7; k++) {
+      const double c = b.q(J.qcol + k);
+      const float v = float(c);
+      small += bfp_small(c);
+      zeros += v == 0.0f;
+      n2 += v * v;
+    }
+    if ((small && small + zeros > 1) || !(n2 > 0.999f && n2 < 1.001f)) b.refuse();
+  } else if (turns(J) && bfp_small(b.q(J.qcol))) {
+    bool aligned = false;
+    for (int k = 0; k < 9; k++) {
+      const i64 r = b.W(b.iR(b.j) + k);
+      aligned = aligned || r > kAligned || r < -kAligned;
+    }
+    if (aligned) b.refuse();
+  }
+}
+// World rotations and positions of all joints into A; refuses what blk_check_configuration does.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_poses(const Blk<A, E, EI>& b) {
   typedef typename A::Vec Vec;
   const DJoint& J = b.J[b.j];
   const BJoint& B = b.B[b.j];
@@ -393,6 +523,7 @@ __device__ __forceinline__ void blk_poses(const Blk<A, E>& b) {
     }
     __syncthreads();
   }
+  blk_check_configuration(b);
   Vec o{};
   if (b.j) {  // offset from the parent's origin
     o = A::offset(J, B);
@@ -428,8 +559,8 @@ __device__ __forceinline__ typename A::Tw column_S(const DJoint& J, const BJoint
 }
 // Motion subspace columns into S and (with_inertia) world inertias into Y, where the joints' own
 // rotations are no longer needed.
-template <class A, int E>
-__device__ __forceinline__ void blk_columns(const Blk<A, E>& b, bool with_inertia) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_columns(const Blk<A, E, EI>& b, bool with_inertia) {
   if (b.col >= 0) {
     const int c = b.col, j = b.col_joint[c];
     b.put(b.L.S + 6 * c, b.L.xS + 2 * c,
@@ -440,8 +571,8 @@ __device__ __forceinline__ void blk_columns(const Blk<A, E>& b, bool with_inerti
   __syncthreads();
 }
 // sum over the slot's joint's columns of v(column of the joint, external column) S
-template <class A, int E, class F>
-__device__ __forceinline__ typename A::Tw joint_motion(const Blk<A, E>& b, const F& v) {
+template <class A, int E, int EI, class F>
+__device__ __forceinline__ typename A::Tw joint_motion(const Blk<A, E, EI>& b, const F& v) {
   const DJoint& J = b.J[b.j];
   typename A::Tw r = norm(mul(A::sc(v(J.ivx, J.vcol)), b.S(J.ivx)));
 #pragma unroll 1
@@ -450,8 +581,8 @@ __device__ __forceinline__ typename A::Tw joint_motion(const Blk<A, E>& b, const
 }
 // The slot's joint's motion m summed from the root (the joint's own on entry), kept at items
 // at(joint) with exponents xat(joint).
-template <class A, int E, class I, class X>
-__device__ __forceinline__ void blk_from_root(const Blk<A, E>& b, typename A::Tw& m, const I& at, const X& xat) {
+template <class A, int E, int EI, class I, class X>
+__device__ __forceinline__ void blk_from_root(const Blk<A, E, EI>& b, typename A::Tw& m, const I& at, const X& xat) {
   if (b.j && b.p == 0) b.put(at(b.j), xat(b.j), m);
   __syncthreads();
 #pragma unroll 1
@@ -464,9 +595,9 @@ __device__ __forceinline__ void blk_from_root(const Blk<A, E>& b, typename A::Tw
   }
 }
 // Velocities (V, by joint), accelerations and body forces (A), with zero joint acceleration
-// unless with_qdd.
-template <class A, int E>
-__device__ __forceinline__ void blk_motion_forces(const Blk<A, E>& b, bool with_qdd) {
+// unless with_qdd; notes the terms of the bias forces, if those are to follow.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_motion_forces(const Blk<A, E, EI>& b, bool with_qdd, bool bias = true) {
   typedef typename A::Tw Tw;
   Tw vj{}, v{}, a{};
   if (b.j) v = vj = joint_motion(b, [&](int, int x) SG_INLINE { return b.qd(x); });
@@ -480,13 +611,16 @@ __device__ __forceinline__ void blk_motion_forces(const Blk<A, E>& b, bool with_
   blk_from_root(b, a, [&](int j) SG_INLINE { return b.iA(j); }, [&](int j) SG_INLINE { return b.xA(j); });
   if (b.j) {
     const typename A::Rbi Y = b.rbi(b.j);
-    b.put_frc(b.j, norm(add(mul(Y, a), crossf(v, norm(mul(Y, v))))));
+    const Tw f = add(mul(Y, a), crossf(v, norm(mul(Y, v))));
+    if constexpr (A::kFixed)  // before norm() an exponent is that of the terms, of about 2^57 each
+      if (bias) b.note(NOTE_SCALE, 57 + (turns(b.J[b.j]) ? f.w.e : f.v.e));
+    b.put_frc(b.j, norm(f));
   }
   __syncthreads();
 }
 // Forces and (composite) inertias summed over subtrees: level by level, each joint its children.
-template <class A, int E>
-__device__ __forceinline__ void blk_subtrees(const Blk<A, E>& b, bool forces, bool composite) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_subtrees(const Blk<A, E, EI>& b, bool forces, bool composite) {
   const int end = b.end[b.j];
   const bool inner = b.j && end > b.j + 1;
 #pragma unroll 1
@@ -510,8 +644,8 @@ __device__ __forceinline__ void blk_subtrees(const Blk<A, E>& b, bool forces, bo
 }
 // Column forces F = Y S (composite Y) into V, M's entries S_c . F_a in FP64 into Y's items
 // (for_output) and M into A as blk_solve takes it (for_solve).
-template <class A, int E>
-__device__ __forceinline__ void blk_mass_matrix(const Blk<A, E>& b, bool for_solve, bool for_output) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_mass_matrix(const Blk<A, E, EI>& b, bool for_solve, bool for_output) {
   typedef typename A::Sc Sc;
   const int c = b.col;
   Sc diag{};
@@ -557,8 +691,8 @@ __device__ __forceinline__ void blk_mass_matrix(const Blk<A, E>& b, bool for_sol
 
 // Pivot of column a: D 4^x in [1/4, 1] and its reciprocal, into the diagonal's word and the
 // pivot shift; a scaled pivot below 2^-40 sends the environment to the FP64 sweep.
-template <class A, int E>
-__device__ __forceinline__ void blk_pivot(const Blk<A, E>& b, int a, int diag) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_pivot(const Blk<A, E, EI>& b, int a, int diag) {
   if constexpr (A::kFixed) {
     const i64 D = b.W(diag);
     if (D < (1LL << 20)) b.refuse();
@@ -570,8 +704,8 @@ __device__ __forceinline__ void blk_pivot(const Blk<A, E>& b, int a, int diag) {
     b.setD(diag, 1.0 / b.D(diag));
   }
 }
-template <class A, int E>
-__device__ __forceinline__ void blk_back(const Blk<A, E>& b);
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_back(const Blk<A, E, EI>& b);
 // M = L^T D L with the right-hand side in b carried along, then x = M^-1 b (after b). By levels
 // from the deepest columns, all columns of a level between two barriers (column by column, with
 // nv of them, 8192 35-DoF humanoids took 366 us instead of 297): slot c updates row c for every
@@ -582,8 +716,8 @@ __device__ __forceinline__ void blk_back(const Blk<A, E>& b);
 // definite matrix has |M_ac| <= sqrt(M_aa M_cc), and so have the matrices that elimination
 // leaves; with D 4^x in [1/4, 1] every h_ac 2^x and f = h_ac 2^x / (D 4^x) stay below 1 and 2,
 // L_ac = f 2^(x_a + s_c - s_a)), or FP64.
-template <class A, int E>
-__device__ __forceinline__ void blk_solve(const Blk<A, E>& b) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_solve(const Blk<A, E, EI>& b) {
   const int nv = b.nv, col = b.col;
   const int row = col >= 0 ? b.L.A + b.row_start[col] : 0, dr = col >= 0 ? b.depth[col] : nv;
   if (dr == b.col_levels - 1) blk_pivot(b, col, row + dr);
@@ -625,8 +759,8 @@ __device__ __forceinline__ void blk_solve(const Blk<A, E>& b) {
   blk_back(b);
 }
 // x = L^-1 x (after b) for L in S / V and D^-1 applied already.
-template <class A, int E>
-__device__ __forceinline__ void blk_back(const Blk<A, E>& b) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_back(const Blk<A, E, EI>& b) {
   const int nv = b.nv;
   const int c = b.slot, dc = c < nv ? b.depth[c] : 0, rc = c < nv ? b.row_start[c] : 0;
   double x = c < nv ? b.D(b.L.b + nv + c) : 0.0;
@@ -641,46 +775,37 @@ __device__ __forceinline__ void blk_back(const Blk<A, E>& b) {
 }
 
 // S_c . (subtree force of the column's joint)
-template <class A, int E>
-__device__ __forceinline__ double blk_torque(const Blk<A, E>& b, int c) {
+template <class A, int E, int EI>
+__device__ __forceinline__ double blk_torque(const Blk<A, E, EI>& b, int c) {
   return A::get(dot(b.S(c), b.frc(b.col_joint[c])));
 }
 
-// qdd (tree columns, at b + nv) = M^-1 (tau - bias) from the inputs in shared memory.
-template <class A, int E>
-__device__ __forceinline__ void blk_forward_dynamics(const Blk<A, E>& b) {
-  blk_poses(b);
+// qdd (tree columns, at b + nv) = M^-1 (tau - bias) from the inputs in shared memory and the poses.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_forward_dynamics(const Blk<A, E, EI>& b) {
   blk_columns(b, true);
   blk_motion_forces(b, false);
   blk_subtrees(b, true, true);
-  if (b.col >= 0)
-    b.setD(b.L.b + b.col, b.tau(b.ext[b.col]) - blk_torque(b, b.col));
+  if (b.col >= 0) {
+    const double h = blk_torque(b, b.col), tau = b.tau(b.ext[b.col]);
+    b.note(NOTE_BIAS, h);
+    b.note(NOTE_DRIVE, tau);
+    b.setD(b.L.b + b.col, tau - h);
+  }
   blk_mass_matrix(b, true, false);
   blk_solve(b);
 }
 
-// Stores an input, with its effect on the environment's flag.
-template <class A, int E>
-__device__ __forceinline__ void blk_in(const Blk<A, E>& b, int at, double v) {
-  b.setD(b.L.in + at, v);
+// Stores an input, with its effect on the environment's notes.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_in(const Blk<A, E, EI>& b, int at, double v) {
+  b.set_in(at, v);
   if (!bfp_fits(v)) b.refuse();
 }
-// After the inputs are in: a free flyer's quaternion off unit length refuses the environment.
-template <class A, int E>
-__device__ __forceinline__ void blk_check_quaternion(const Blk<A, E>& b) {
-  if (b.j && b.J[b.j].kind == JK_FREEFLYER) {
-    float n2 = 0;
-    for (int k = 3; k < 7; k++) {
-      const float v = float(b.q(b.J[b.j].qcol + k));
-      n2 += v * v;
-    }
-    if (!(n2 > 0.999f && n2 < 1.001f)) b.refuse();
-  }
-}
-// Reads the environment's inputs; whether they suit BfpAlg goes to its flag.
-template <class A, int E>
-__device__ __forceinline__ void blk_load(const Blk<A, E>& b, int ops, const StepArgs& args, int64_t e) {
-  if (b.slot == 0) b.X(b.L.ints - 1) = 0;
+// Reads the environment's inputs; whether they suit BfpAlg goes to its notes.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_load(const Blk<A, E, EI>& b, int ops, const StepArgs& args, int64_t e) {
+  b.clear_notes(0);
   __syncthreads();
 #pragma unroll 1
   for (int c = b.slot; c < b.nq; c += b.slots) blk_in(b, c, ldv(args.q, e, c));
@@ -691,13 +816,12 @@ __device__ __forceinline__ void blk_load(const Blk<A, E>& b, int ops, const Step
     if (ops & OP_ABA) blk_in(b, b.nq + 2 * b.nv + c, ldv(args.tau, e, c));
   }
   __syncthreads();
-  blk_check_quaternion(b);
 }
 
 // Semi-implicit Euler in place on the environment's rows of q and qd (args.q, args.qd) from the
 // inputs in shared memory and qdd at b + nv, as hetero_integrate_kernel does it.
-template <class A, int E>
-__device__ __forceinline__ void blk_euler_rows(const Blk<A, E>& b, const StepArgs& args, int64_t e, double dt) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_euler_rows(const Blk<A, E, EI>& b, const StepArgs& args, int64_t e, double dt) {
   if (!b.j) return;
   const DJoint& J = b.J[b.j];
   double v[6], q[7];
@@ -716,21 +840,20 @@ __device__ __forceinline__ void blk_euler_rows(const Blk<A, E>& b, const StepArg
   }
 }
 
-// One sweep over the block's environments, rows row(0 .. envs - 1) of the arrays (this thread's:
-// e); results are written for those with want(environment in block).
-template <class A, int E, class Row, class Want>
-__device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const StepArgs& args, int64_t e, const Row& row,
-                                         int envs, const Want& want) {
+// One sweep over the block's environments, whose poses are there; row(environment in block): its row of the arrays,
+// this thread's e.
+template <class A, int E, int EI, class Row>
+__device__ __forceinline__ void blk_step(const Blk<A, E, EI>& b, int ops, const StepArgs& args, int64_t e,
+                                         const Row& row) {
   typedef typename A::Sc Sc;
   typedef typename A::Vec Vec;
   typedef typename A::Rot Rot;
-  const bool valid = b.lane < envs && want(b.lane);
+  const bool valid = b.valid;
   // (run-time flags, uniform in the grid: one kernel per E serves every op set)
   const bool kFK = ops & OP_FK, kJAC = ops & OP_JAC, kCRBA = ops & OP_CRBA, kRNEA = ops & OP_RNEA,
              kABA = ops & OP_ABA;
   const bool kVel = kRNEA || kABA, kComposite = kCRBA || kABA, kInertia = kVel || kCRBA;
   const int nv = b.nv;
-  blk_poses(b);
   if (kFK) {
     const DLink* LT = model_links(b.m);
     const BLink* BL = model_blinks(b.m);
@@ -772,6 +895,7 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
   blk_subtrees(b, kVel, kComposite);
   if (kVel && c >= 0) {
     const double f = blk_torque(b, c);
+    b.note(NOTE_BIAS, f);
     if (kABA) b.setD(b.L.b + c, f);
     else if (valid) stv(args.tau_out, e, xc, f);
   }
@@ -788,8 +912,7 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
     for (int rc = threadIdx.x; rc < nv * nv; rc += blockDim.x) {
       const int i = b.pair_of[rc];
 #pragma unroll 1
-      for (int el = 0; el < envs; el++)
-        if (want(el)) stv(args.M, row(el), rc, i < 0 ? 0.0 : __longlong_as_double(b.w[(b.L.Y + i) * E + el]));
+      for (int l = 0; l < b.count; l++) stv(args.M, row(b.env_at(l)), rc, i < 0 ? 0.0 : b.D(b.L.Y + i, l));
     }
   }
   if (!kABA) return;
@@ -803,8 +926,10 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
         const int i = of[k];
         if (i >= 0) t = fma(b.D(b.L.Y + i), b.qdd(k), t);
       }
+      b.note(NOTE_TORQUE, t);
       if (valid) stv(args.tau_out, e, xc, t);
     }
+    b.note(NOTE_DRIVE, b.tau(xc));
     b.setD(b.L.b + c, b.tau(xc) - h);
   }
   __syncthreads();
@@ -816,49 +941,56 @@ __device__ __forceinline__ void blk_step(const Blk<A, E>& b, int ops, const Step
 }  // namespace bfp
 
 #ifdef __CUDACC__
-// (at most 640 threads, so that a thread may hold 96 registers)
-// Runs body(block state, valid) in block floating point, and again in FP64 for the environments
-// that refused (valid then holds for those only).
-template <int E, class F>
-__device__ __forceinline__ void blk_run(const DModel* model, long long* smem, bool adjoint, int envs, const F& body) {
+// Runs body(block state) in block floating point on the block's `envs` environments, whose inputs
+// load(block state) has read and whose poses are there, and in FP64 for those that refused (lost:
+// see Blk::refused). Only these are repeated, packed side by side, and block floating point goes
+// no further than the poses where all refuse. CRBA + RNEA + forward dynamics of 16384 9-DoF arms,
+// with the call: 112 us with none refused, 150 with 8, 192 with 1 in 20, 203 with all (131072: 584,
+// 584, 1178, 1166); before, with the whole block repeated, 158, 251 and 257 (585, 1484, 1509).
+template <int E, class Ld, class F>
+__device__ __forceinline__ void blk_run(const DModel* model, long long* smem, bool adjoint, int envs, int lost,
+                                        const Ld& load, const F& body) {
   bfp::Blk<bfp::BfpAlg, E> b;
-  b.init(model, smem, adjoint);
-  if (b.slot == 0) b.X(b.L.ints - 1) = 0;
-  __syncthreads();
-  body(b, b.lane < envs);
-  __syncthreads();
-  const int refused = b.X(b.L.ints - 1);
-  if (__syncthreads_or(refused)) {
-    bfp::Blk<bfp::FpAlg, E> f;
-    f.init(model, smem, adjoint);
-    __syncthreads();
-    body(f, f.lane < envs && refused);
+  b.init(model, smem, envs, adjoint);
+  load(b);
+  bfp::blk_poses(b);
+  const bool none = __syncthreads_and(b.note_at(0, bfp::NOTE_REFUSED));
+  if (!none) body(b);
+  __syncthreads();  // all notes are in
+  if (__syncthreads_or(none || b.refused(lost))) {
+    unsigned which = 0;
+    for (int k = 0; k < envs; k++) {
+      b.el = k;
+      which |= unsigned(none || b.refused(lost)) << k;
+    }
+    if (which == 0) return;  // (a lane beyond the batch repeats the last environment)
+    bfp::Blk<bfp::FpAlg, 0, E> f;
+    f.init_some(model, smem, which, 0, adjoint);
+    bfp::blk_poses(f);
+    body(f);
   }
 }
 
 // ROWS: the environments are rows of the arrays by a list, and may take an Euler step (an
-// instantiation of its own: the plain sweep is 4 % slower with it).
+// instantiation of its own: the plain sweep is 4 % slower with it). At most 640 threads, so that
+// a thread may hold 96 registers.
 template <int E, bool ROWS>
 __global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_block_kernel(const DModel* __restrict__ model, int ops,
                                                                         const StepArgs args, const BfpRows r) {
   extern __shared__ __align__(16) long long smem[];
-  bfp::Blk<bfp::BfpAlg, E> b;
-  b.init(model, smem);
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = args.n - e0 < E ? int(args.n - e0) : E;
-  auto row = [&](int el) SG_INLINE { return ROWS ? int64_t(r.rows[e0 + el]) : e0 + el; };
-  const int64_t e = row(b.lane < envs ? b.lane : envs - 1);
-  bfp::blk_load(b, ops, args, e);
-  bfp::blk_step(b, ops, args, e, row, envs, [](int) { return true; });
-  const int refused = b.X(b.L.ints - 1);
-  if (ROWS && r.integrate && b.lane < envs && !refused) bfp::blk_euler_rows(b, args, e, r.dt);
-  if (__syncthreads_or(refused)) {  // FP64 for the environments that the sweep above turned away
-    bfp::Blk<bfp::FpAlg, E> f;
-    f.init(model, smem);
-    const int* flag = f.x + (f.L.ints - 1) * E;
-    bfp::blk_step(f, ops, args, e, row, envs, [&](int lane) SG_INLINE { return flag[lane] != 0; });
-    if (ROWS && r.integrate && f.lane < envs && refused) bfp::blk_euler_rows(f, args, e, r.dt);
-  }
+  auto row = [&](int el) SG_INLINE {
+    const int64_t e = e0 + min(el, envs - 1);
+    return ROWS ? int64_t(r.rows[e]) : e;
+  };
+  blk_run<E>(
+      model, smem, false, envs, bfp::kLost, [&](auto& b) SG_INLINE { bfp::blk_load(b, ops, args, row(b.el)); },
+      [&](auto& b) SG_INLINE {
+        const int64_t e = row(b.el);
+        bfp::blk_step(b, ops, args, e, row);
+        if (ROWS && r.integrate && b.valid && !b.refused()) bfp::blk_euler_rows(b, args, e, r.dt);
+      });
 }
 
 // PhysxArticulation::computePassiveForce on float32 state rows (physx_interop.cu): RNEA at zero
@@ -869,21 +1001,29 @@ __global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_passive_kernel(const 
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, false, envs, [&](auto& b, bool valid) SG_INLINE {
-    const int64_t e = e0 + min(b.lane, envs - 1);
-    if (!a.gravity) b.g[0] = b.g[1] = b.g[2] = 0.0;
-    if (b.col >= 0) {  // one-DoF joints only: as many coordinates as columns
-      bfp::blk_in(b, b.col, double(a.qpos[e * a.in_stride + b.col]));
-      bfp::blk_in(b, b.nq + b.col, a.coriolis ? double(a.qvel[e * a.in_stride + b.col]) : 0.0);
-    }
-    __syncthreads();
-    bfp::blk_poses(b);
-    bfp::blk_columns(b, true);
-    bfp::blk_motion_forces(b, false);
-    bfp::blk_subtrees(b, true, false);
-    if (b.col >= 0 && valid)
-      a.qf[e * a.out_stride + b.ext[b.col]] = float(bfp::blk_torque(b, b.col));
-  });
+  blk_run<E>(
+      model, smem, false, envs, bfp::kLostFloat,
+      [&](auto& b) SG_INLINE {
+        const int64_t e = e0 + min(b.el, envs - 1);
+        b.clear_notes(0);
+        __syncthreads();
+        if (b.col >= 0) {  // one-DoF joints only: as many coordinates as columns
+          bfp::blk_in(b, b.col, double(a.qpos[e * a.in_stride + b.col]));
+          bfp::blk_in(b, b.nq + b.col, a.coriolis ? double(a.qvel[e * a.in_stride + b.col]) : 0.0);
+        }
+        __syncthreads();
+      },
+      [&](auto& b) SG_INLINE {
+        if (!a.gravity) b.g[0] = b.g[1] = b.g[2] = 0.0;
+        bfp::blk_columns(b, true);
+        bfp::blk_motion_forces(b, false);
+        bfp::blk_subtrees(b, true, false);
+        if (b.col >= 0) {
+          const double f = bfp::blk_torque(b, b.col);
+          b.note(bfp::NOTE_BIAS, f);
+          if (b.valid) a.qf[(e0 + b.el) * a.out_stride + b.ext[b.col]] = float(f);
+        }
+      });
 }
 
 // Launches a kernel with `smem` bytes of dynamic shared memory.

@@ -39,112 +39,152 @@ static __device__ __noinline__ void ff_integrate_adjoint(const double* d, double
   vb[0] = v.v.x; vb[1] = v.v.y; vb[2] = v.v.z; vb[3] = v.w.x; vb[4] = v.w.y; vb[5] = v.w.z;
 }
 
-// Whether the environment is left to the FP64 pass that follows: its results are not written,
-// they may lie where that pass reads its inputs.
-template <class A, int E>
-__device__ __forceinline__ bool blk_refused(const Blk<A, E>& b) {
-  return A::kFixed && b.X(b.L.ints - 1) != 0;
-}
 // 1 / D of column c after blk_solve.
-template <class A, int E>
-__device__ __forceinline__ double blk_inverse_pivot(const Blk<A, E>& b, int c) {
+template <class A, int E, int EI>
+__device__ __forceinline__ double blk_inverse_pivot(const Blk<A, E, EI>& b, int c) {
   const int i = b.L.A + b.row_start[c] + b.depth[c];
   if constexpr (A::kFixed) return to_double(b.W(i), 2 * b.X(b.L.xs + b.nv + c) - 58 - 2 * b.X(b.L.xs + c));
   else return b.D(i);
 }
-// Semi-implicit Euler on the inputs in shared memory with qdd at b + nv.
-template <class A, int E>
-__device__ __forceinline__ void blk_integrate(const Blk<A, E>& b, double dt) {
-  if (b.col >= 0) {
-    const int x = b.ext[b.col];
-    blk_in(b, b.nq + x, fma(dt, b.D(b.L.b + b.nv + b.col), b.qd(x)));
+// Semi-implicit Euler on the inputs in shared memory with qdd at b + nv, in two parts with a
+// barrier between: velocities, then coordinates.
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_integrate_velocity(const Blk<A, E, EI>& b, double dt) {
+  if (b.col < 0) return;
+  const int x = b.ext[b.col];
+  b.set_in(b.nq + x, fma(dt, b.D(b.L.b + b.nv + b.col), b.qd(x)));
+}
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_integrate_position(const Blk<A, E, EI>& b, double dt) {
+  if (!b.j) return;
+  const DJoint& J = b.J[b.j];
+  if (J.kind == JK_FREEFLYER) {
+    double q[7], d[6];
+    for (int k = 0; k < 7; k++) q[k] = b.q(J.qcol + k);
+    for (int k = 0; k < 6; k++) d[k] = b.qd(J.vcol + k);
+    free_flyer_step(q, d, dt);
+    for (int k = 0; k < 7; k++) b.set_in(J.qcol + k, q[k]);
+  } else {
+    b.set_in(J.qcol, fma(dt, b.qd(J.vcol), b.q(J.qcol)));
   }
-  __syncthreads();
-  if (b.j) {
-    const DJoint& J = b.J[b.j];
-    if (J.kind == JK_FREEFLYER) {
-      double q[7], d[6];
-      for (int k = 0; k < 7; k++) q[k] = b.q(J.qcol + k);
-      for (int k = 0; k < 6; k++) d[k] = b.qd(J.vcol + k);
-      free_flyer_step(q, d, dt);
-      for (int k = 0; k < 7; k++) blk_in(b, J.qcol + k, q[k]);
-    } else {
-      blk_in(b, J.qcol, fma(dt, b.qd(J.vcol), b.q(J.qcol)));
-    }
-  }
-  __syncthreads();
 }
 // A row of an env-major state into the inputs.
-template <class A, int E>
-__device__ __forceinline__ void blk_load_row(const Blk<A, E>& b, int at, const double* row, int cols) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_load_row(const Blk<A, E, EI>& b, int at, const double* row, int cols) {
 #pragma unroll 1
-  for (int c = b.slot; c < cols; c += b.slots) blk_in(b, at + c, row[c]);
+  for (int c = b.slot; c < cols; c += b.slots) b.set_in(at + c, row[c]);
 }
 
-// T steps (from step t0 on) for the block's environments; per step record(t) before it and
-// after(t) when qdd is at b + nv.
-template <class A, int E, class R, class F>
-__device__ __forceinline__ void blk_steps(const Blk<A, E>& b, const RolloutArgs& a, int64_t e, int t0, int t1,
-                                          const R& record, const F& after) {
-  const int at = b.nq + 2 * b.nv;
+// The environments of the block that refused, from every thread of it.
+template <int E>
+__device__ __forceinline__ unsigned blk_refused_set(Blk<BfpAlg, E>& b) {
+  unsigned which = 0;
+  const int el = b.el;
+  for (int k = 0; k < b.count; k++) {
+    b.el = k;
+    which |= unsigned(b.refused()) << k;
+  }
+  b.el = el;
+  return which;
+}
+// Steps t0 to t1 - 1 of the block's environments, whose q and qd are among the inputs; per step
+// record(block state, t) before it and after(block state, t) when qdd is at b + nv. A step in FP64
+// for the environments that refuse it alone: the next one is asked again.
+template <int E, class R, class F>
+__device__ __forceinline__ void blk_steps(Blk<BfpAlg, E>& b, const DModel* model, long long* smem, const RolloutArgs& a,
+                                          int64_t e, int t0, int t1, const R& record, const F& after) {
+  const int nq = b.nq, nv = b.nv;
+  b.clear_notes(0);
+  b.set = 0;
+  __syncthreads();
 #pragma unroll 1
   for (int t = t0; t < t1; t++) {
-    record(t);
-    blk_load_row(b, at, a.tau + (int64_t(t) * a.n + e) * b.nv, b.nv);
+    record(b, t);
+    const double* tau = a.tau + (int64_t(t) * a.n + e) * nv;
+#pragma unroll 1
+    for (int c = b.slot; c < nv; c += b.slots) {
+      blk_in(b, nq + 2 * nv + c, tau[c]);
+      if (!bfp_fits(b.qd(c))) b.refuse();
+    }
+#pragma unroll 1
+    for (int c = b.slot; c < nq; c += b.slots)
+      if (!bfp_fits(b.q(c))) b.refuse();
     __syncthreads();
-    blk_forward_dynamics(b);
-    after(t);
-    blk_integrate(b, a.dt);
+    b.clear_notes(b.set ^ 1);
+    blk_poses(b);
+    const bool none = __syncthreads_and(b.note_at(b.set, NOTE_REFUSED));
+    if (!none) {
+      blk_forward_dynamics(b);
+      after(b, t);
+      if (!b.refused()) blk_integrate_velocity(b, a.dt);
+    }
+    const bool some = __syncthreads_or(none || b.refused());
+    if (!none && !b.refused()) blk_integrate_position(b, a.dt);
+    if (some) {
+      const unsigned which = blk_refused_set(b);
+      if (which) {
+        Blk<FpAlg, 0, E> f;
+        f.init_some(model, smem, which, b.set);
+        blk_poses(f);
+        blk_forward_dynamics(f);
+        after(f, t);
+        if (f.valid) blk_integrate_velocity(f, a.dt);
+        __syncthreads();
+        if (f.valid) blk_integrate_position(f, a.dt);
+      }
+    }
+    b.set ^= 1;
+    __syncthreads();
   }
 }
 
-template <class A, int E>
-__device__ __forceinline__ void blk_rollout(const Blk<A, E>& b, const RolloutArgs& a, int64_t e, bool valid) {
+template <int E>
+__device__ __forceinline__ void blk_rollout(Blk<BfpAlg, E>& b, const DModel* model, long long* smem,
+                                            const RolloutArgs& a, int64_t e) {
   const int64_t n = a.n;
   const int nq = b.nq, nv = b.nv;
   blk_load_row(b, 0, a.q0 + e * nq, nq);
   blk_load_row(b, nq, a.qd0 + e * nv, nv);
-  __syncthreads();
-  blk_check_quaternion(b);
   auto put = [&](double* q, double* qd) SG_INLINE {
-    if (!valid) return;
+    if (!b.valid) return;
 #pragma unroll 1
     for (int c = b.slot; c < nq; c += b.slots) q[e * nq + c] = b.q(c);
 #pragma unroll 1
     for (int c = b.slot; c < nv; c += b.slots) qd[e * nv + c] = b.qd(c);
   };
   blk_steps(
-      b, a, e, 0, a.T,
-      [&](int t) SG_INLINE {
+      b, model, smem, a, e, 0, a.T,
+      [&](const auto&, int t) SG_INLINE {
         if (a.q_ckpt && t % a.K == 0) put(a.q_ckpt + int64_t(t / a.K) * n * nq, a.qd_ckpt + int64_t(t / a.K) * n * nv);
       },
-      [](int) {});
-  if (!blk_refused(b)) put(a.qT, a.qdT);
+      [](const auto&, int) {});
+  put(a.qT, a.qdT);
 }
 
 // One segment: its steps' records into the scratch ([segment of group][step][field][env]).
-template <class A, int E>
-__device__ __forceinline__ void blk_replay(const Blk<A, E>& b, const RolloutArgs& a, int g, int64_t e, bool valid) {
+template <int E>
+__device__ __forceinline__ void blk_replay(Blk<BfpAlg, E>& b, const DModel* model, long long* smem,
+                                           const RolloutArgs& a, int g, int64_t e0, int64_t e) {
   const int64_t n = a.n;
   const int nq = b.nq, nv = b.nv, s = a.s_lo + g;
   const int64_t rec = blk_record_doubles(nv, nq, b.npairs);
   blk_load_row(b, 0, a.q_ckpt + (int64_t(s) * n + e) * nq, nq);
   blk_load_row(b, nq, a.qd_ckpt + (int64_t(s) * n + e) * nv, nv);
-  __syncthreads();
-  blk_check_quaternion(b);
   const int t0 = s * a.K, t1 = min(a.T, t0 + a.K);
-  auto base = [&](int t) SG_INLINE { return a.scratch + (int64_t(g) * a.K + (t - t0)) * rec * n + e; };
+  auto base = [&](const auto& c, int t) SG_INLINE {
+    return a.scratch + (int64_t(g) * a.K + (t - t0)) * rec * n + e0 + c.el;
+  };
   blk_steps(
-      b, a, e, t0, t1,
-      [&](int t) SG_INLINE {
-        if (!valid) return;
-        double* o = base(t);
+      b, model, smem, a, e, t0, t1,
+      [&](const auto& b, int t) SG_INLINE {
+        if (!b.valid) return;
+        double* o = base(b, t);
 #pragma unroll 1
-        for (int c = b.slot; c < nq + nv; c += b.slots) o[c * n] = b.D(b.L.in + c);
+        for (int c = b.slot; c < nq + nv; c += b.slots) o[c * n] = b.in(c);
       },
-      [&](int t) SG_INLINE {
-        if (!valid) return;
-        double* o = base(t) + (nq + nv) * n;
+      [&](const auto& b, int t) SG_INLINE {
+        if (!b.valid) return;
+        double* o = base(b, t) + (nq + nv) * n;
         if (b.col >= 0) {
           o[b.ext[b.col] * n] = b.D(b.L.b + nv + b.col);
           o[int64_t(nv + b.row_start[b.col] + b.depth[b.col]) * n] = blk_inverse_pivot(b, b.col);
@@ -156,8 +196,8 @@ __device__ __forceinline__ void blk_replay(const Blk<A, E>& b, const RolloutArgs
 }
 
 // x = M^-1 b for the factor in Y's items (1 / D on the diagonal), b at L.b, x after it.
-template <class A, int E>
-__device__ __forceinline__ void blk_factor_solve(const Blk<A, E>& b) {
+template <class A, int E, int EI>
+__device__ __forceinline__ void blk_factor_solve(const Blk<A, E, EI>& b) {
   const int nv = b.nv, c = b.col;
   const int dc = c >= 0 ? b.depth[c] : 0, rc = c >= 0 ? b.row_start[c] : 0;
   double y = c >= 0 ? b.D(b.L.b + c) : 0.0;  // L^T y = b, deepest columns first
@@ -188,14 +228,13 @@ __device__ __forceinline__ void blk_factor_solve(const Blk<A, E>& b) {
   }
 }
 
-// RNEA adjoint at the inputs q, qd, qdd in shared memory for the adjoint lam (tree columns) at
-// b + nv: out(column, qbar, qdbar, qddbar), unscaled.
-template <class A, int E, class F>
-__device__ __forceinline__ void blk_rnea_adjoint(const Blk<A, E>& b, const F& out) {
+// RNEA adjoint at the inputs q, qd, qdd in shared memory and the poses, for the adjoint lam (tree
+// columns) at b + nv: out(column, qbar, qdbar, qddbar), unscaled.
+template <class A, int E, int EI, class F>
+__device__ __forceinline__ void blk_rnea_adjoint(const Blk<A, E, EI>& b, const F& out) {
   typedef typename A::Tw Tw;
-  blk_poses(b);
   blk_columns(b, true);
-  blk_motion_forces(b, true);
+  blk_motion_forces(b, true, false);
   blk_subtrees(b, true, false);
   // w = sum of lam S from the root, into u
   Tw w{};
@@ -236,25 +275,32 @@ __device__ __forceinline__ void blk_rnea_adjoint(const Blk<A, E>& b, const F& ou
   }
   if (b.j) {
     const DJoint& J = b.J[b.j];
-    Tw G{};
+    Tw G{}, terms{};
     const bool root = b.p == 0;
     if (root) {  // G = v_p x* (v_p x* P - X) - a_p x* P - w_p x* F
       Tw a{};
       a.v = A::vec(-b.g[0], -b.g[1], -b.g[2]);
       a.w = A::vec(0, 0, 0);
-      G = norm(neg(crossf(a, P)));
+      const Tw t = crossf(a, P);
+      if constexpr (A::kFixed) terms = t;
+      G = norm(neg(t));
     } else {
       const Tw vp = b.V(b.p - 1), wp = b.tw(b.L.u + 6 * (b.p - 1), b.L.xu + 2 * (b.p - 1));
+      const Tw t = crossf(b.acc(b.p), P), u = crossf(wp, b.frc(b.j));
       G = norm(add(norm(crossf(vp, P)), neg(X)));
-      G = norm(add(norm(crossf(vp, G)), neg(norm(crossf(b.acc(b.p), P)))));
-      G = norm(add(G, neg(norm(crossf(wp, b.frc(b.j))))));
+      G = norm(add(norm(crossf(vp, G)), neg(norm(t))));
+      G = norm(add(G, neg(norm(u))));
+      if constexpr (A::kFixed) terms = add(t, u);
       v = norm(add(vp, v));
     }
+    if constexpr (A::kFixed) b.note(NOTE_GSCALE, 57 + (turns(J) ? terms.w.e : terms.v.e));
     const Tw Gd = norm(add(X, neg(norm(crossf(v, P)))));
 #pragma unroll 1
     for (int k = 0; k < J.nv; k++) {
       const Tw S = b.S(J.ivx + k);
-      out(J.ivx + k, 0, A::get(dot(S, G)));
+      const double gq = A::get(dot(S, G));
+      b.note(NOTE_GRAD, gq);
+      out(J.ivx + k, 0, gq);
       out(J.ivx + k, 1, A::get(dot(S, Gd)));
       out(J.ivx + k, 2, A::get(dot(S, P)));
     }
@@ -262,10 +308,79 @@ __device__ __forceinline__ void blk_rnea_adjoint(const Blk<A, E>& b, const F& ou
   __syncthreads();
 }
 
-// Reverse pass of a group of segments, latest step first. Each slot keeps its column's entries of
-// the state's adjoint in registers (a free flyer's tangent block: six slots).
-template <class A, int E>
-__device__ __forceinline__ void blk_reverse(const Blk<A, E>& b, const RolloutArgs& a, int64_t e, bool valid) {
+// One step of the reverse pass, record r of it (field stride n) and the state's adjoint (tangent
+// layout, tree columns: q's then qd's) in the place of tau and on, replaced by that before the step.
+// refused(): whether to leave it to another pass.
+template <class A, int E, int EI, class P>
+__device__ __forceinline__ void blk_reverse_step(const Blk<A, E, EI>& b, const RolloutArgs& a, const double* r,
+                                                 double* tau_bar, const P& refused) {
+  const int64_t n = a.n;
+  const int nq = b.nq, nv = b.nv, c = b.col;
+  const int jc = c >= 0 ? b.col_joint[c] : 1, x = c >= 0 ? b.ext[c] : 0;
+  const bool ff = c >= 0 && b.J[jc].kind == JK_FREEFLYER;
+  const int at = nq + 2 * nv + c;
+  double qb = c >= 0 ? b.in(at) : 0.0, qdb = c >= 0 ? b.in(at + nv) : 0.0;
+#pragma unroll 1
+  for (int k = b.slot; k < nq + 2 * nv; k += b.slots) blk_in(b, k, r[k * n]);
+#pragma unroll 1
+  for (int k = b.slot; k < b.npairs; k += b.slots) b.setD(b.L.Y + k, r[(nq + 2 * nv + int64_t(k)) * n]);
+  // q' = q (+) dt qd', qd' = qd + dt qdd, reversed
+  if (c >= 0 && !ff) qdb = fma(a.dt, qb, qdb);
+  if (ff) {  // the block of six at once: through b
+    b.setD(b.L.b + c, qb);
+    b.setD(b.L.b + nv + c, qdb);
+  }
+  __syncthreads();
+  if (ff && b.col_dof[c] == 0) {
+    double d[6], g[6], vb[6];
+    for (int k = 0; k < 6; k++) {
+      d[k] = a.dt * fma(a.dt, b.qdd(x + k), b.qd(x + k));  // the step's displacement
+      g[k] = b.D(b.L.b + c + k);
+      vb[k] = b.D(b.L.b + nv + c + k);
+    }
+    ff_integrate_adjoint(d, a.dt, g, vb);
+    for (int k = 0; k < 6; k++) {
+      b.setD(b.L.b + c + k, g[k]);
+      b.setD(b.L.b + nv + c + k, vb[k]);
+    }
+  }
+  __syncthreads();
+  if (ff) {
+    qb = b.D(b.L.b + c);
+    qdb = b.D(b.L.b + nv + c);
+  }
+  if (c >= 0) b.setD(b.L.b + c, a.dt * qdb);
+  __syncthreads();
+  blk_factor_solve(b);  // lam at b + nv
+  if (c >= 0) {
+    const double lam = b.D(b.L.b + nv + c);
+    if (!bfp_fits(lam)) b.refuse();
+    if (b.valid) tau_bar[x] = lam;
+  }
+  blk_poses(b);
+  blk_rnea_adjoint(b, [&](int col, int which, double v) SG_INLINE {
+    if (which < 2) b.setD(b.L.b + (which == 0 ? 0 : nv) + col, v);
+  });
+  if (c >= 0 && !refused()) {
+    b.set_in(at, qb - b.D(b.L.b + c));
+    b.set_in(at + nv, qdb - b.D(b.L.b + nv + c));
+  }
+}
+
+// In FP64 for the environments in `which` (a call of its own: inlined, its registers cost the
+// reverse pass 330 more bytes of spills).
+template <int E>
+__device__ __noinline__ void blk_reverse_step_fp64(const DModel* model, long long* smem, unsigned which, int set,
+                                                   const RolloutArgs a, const double* r, double* tau_bar) {
+  Blk<FpAlg, 0, E> f;
+  f.init_some(model, smem, which, set, true);
+  blk_reverse_step(f, a, r + f.el, tau_bar + int64_t(f.el) * f.nv, [&]() SG_INLINE { return !f.valid; });
+}
+// Reverse pass of a group of segments, latest step first; a step in FP64 for the environments
+// that refuse it.
+template <int E>
+__device__ __forceinline__ void blk_reverse(Blk<BfpAlg, E>& b, const DModel* model, long long* smem,
+                                            const RolloutArgs& a, int64_t e0, int64_t e) {
   const int64_t n = a.n;
   const int nq = b.nq, nv = b.nv;
   const int64_t rec = blk_record_doubles(nv, nq, b.npairs);
@@ -277,70 +392,33 @@ __device__ __forceinline__ void blk_reverse(const Blk<A, E>& b, const RolloutArg
   const int c = b.col;
   const int jc = c >= 0 ? b.col_joint[c] : 1, x = c >= 0 ? b.ext[c] : 0;
   const int qx = c >= 0 ? b.J[jc].qcol + b.col_dof[c] : 0;
-  const bool ff = c >= 0 && b.J[jc].kind == JK_FREEFLYER;
-  double qb = c >= 0 && qin ? qin[e * nq + qx] : 0.0, qdb = c >= 0 && qdin ? qdin[e * nv + x] : 0.0;
-  auto check = [&](double v) SG_INLINE {
-    if (!bfp_fits(v)) b.refuse();
-  };
+  if (c >= 0) {
+    b.set_in(nq + 2 * nv + c, qin ? qin[e * nq + qx] : 0.0);
+    b.set_in(nq + 3 * nv + c, qdin ? qdin[e * nv + x] : 0.0);
+  }
+  b.clear_notes(0);
+  __syncthreads();
 #pragma unroll 1
   for (int s = a.s_lo + a.s_cnt - 1; s >= a.s_lo; s--) {
     const int t0 = s * a.K, t1 = min(a.T, t0 + a.K);
 #pragma unroll 1
     for (int t = t1 - 1; t >= t0; t--) {
-      const double* r = a.scratch + (int64_t(s - a.s_lo) * a.K + (t - t0)) * rec * n + e;
-#pragma unroll 1
-      for (int k = b.slot; k < nq + 2 * nv; k += b.slots) blk_in(b, k, r[k * n]);
-#pragma unroll 1
-      for (int k = b.slot; k < b.npairs; k += b.slots) b.setD(b.L.Y + k, r[(nq + 2 * nv + int64_t(k)) * n]);
-      // q' = q (+) dt qd', qd' = qd + dt qdd, reversed
-      if (c >= 0 && !ff) qdb = fma(a.dt, qb, qdb);
-      if (ff) {  // the block of six at once: through b
-        b.setD(b.L.b + c, qb);
-        b.setD(b.L.b + nv + c, qdb);
+      const double* r = a.scratch + (int64_t(s - a.s_lo) * a.K + (t - t0)) * rec * n;
+      double* tau_bar = a.tau_bar + int64_t(t) * n * nv;
+      b.clear_notes(b.set ^ 1);
+      blk_reverse_step(b, a, r + e, tau_bar + e * nv, [&]() SG_INLINE { return b.refused(); });
+      if (__syncthreads_or(b.refused())) {
+        if (const unsigned which = blk_refused_set(b))
+          blk_reverse_step_fp64<E>(model, smem, which, b.set, a, r + e0, tau_bar + e0 * nv);
       }
-      __syncthreads();
-      if (ff && b.col_dof[c] == 0) {
-        double d[6], g[6], vb[6];
-        for (int k = 0; k < 6; k++) {
-          d[k] = a.dt * fma(a.dt, b.qdd(x + k), b.qd(x + k));  // the step's displacement
-          g[k] = b.D(b.L.b + c + k);
-          vb[k] = b.D(b.L.b + nv + c + k);
-        }
-        ff_integrate_adjoint(d, a.dt, g, vb);
-        for (int k = 0; k < 6; k++) {
-          b.setD(b.L.b + c + k, g[k]);
-          b.setD(b.L.b + nv + c + k, vb[k]);
-        }
-      }
-      __syncthreads();
-      if (ff) {
-        qb = b.D(b.L.b + c);
-        qdb = b.D(b.L.b + nv + c);
-      }
-      if (c >= 0) b.setD(b.L.b + c, a.dt * qdb);
-      __syncthreads();
-      blk_factor_solve(b);  // lam at b + nv
-      if (c >= 0) {
-        const double lam = b.D(b.L.b + nv + c);
-        check(lam);
-        if (valid) a.tau_bar[(int64_t(t) * n + e) * nv + x] = lam;
-      }
-      blk_rnea_adjoint(b, [&](int col, int which, double v) SG_INLINE {
-        if (which < 2) b.setD(b.L.b + (which == 0 ? 0 : nv) + col, v);
-      });
-      if (c >= 0) {
-        qb -= b.D(b.L.b + c);
-        qdb -= b.D(b.L.b + nv + c);
-        check(qb);
-        check(qdb);
-      }
+      b.set ^= 1;
       __syncthreads();
     }
   }
-  if (c >= 0 && valid && !blk_refused(b)) {
-    a.q0_bar[e * nq + qx] = qb;
-    a.qd0_bar[e * nv + x] = qdb;
-    if (ff && b.col_dof[c] == 0) a.q0_bar[e * nq + qx + 6] = 0.0;
+  if (c >= 0 && b.valid) {
+    a.q0_bar[e * nq + qx] = b.in(nq + 2 * nv + c);
+    a.qd0_bar[e * nv + x] = b.in(nq + 3 * nv + c);
+    if (b.J[jc].kind == JK_FREEFLYER && b.col_dof[c] == 0) a.q0_bar[e * nq + qx + 6] = 0.0;
   }
 }
 #endif  // __CUDACC__
@@ -354,9 +432,9 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_rollout_kernel(const
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, false, envs, [&](const auto& b, bool valid) SG_INLINE {
-    bfp::blk_rollout(b, a, e0 + min(b.lane, envs - 1), valid);
-  });
+  bfp::Blk<bfp::BfpAlg, E> b;
+  b.init(model, smem, envs);
+  bfp::blk_rollout(b, model, smem, a, e0 + min(b.el, envs - 1));
 }
 template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_replay_kernel(const DModel* __restrict__ model,
@@ -364,9 +442,9 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_replay_kernel(const 
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, false, envs, [&](const auto& b, bool valid) SG_INLINE {
-    bfp::blk_replay(b, a, int(blockIdx.y), e0 + min(b.lane, envs - 1), valid);
-  });
+  bfp::Blk<bfp::BfpAlg, E> b;
+  b.init(model, smem, envs);
+  bfp::blk_replay(b, model, smem, a, int(blockIdx.y), e0, e0 + min(b.el, envs - 1));
 }
 template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_reverse_kernel(const DModel* __restrict__ model,
@@ -374,11 +452,28 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_reverse_kernel(const
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, true, envs, [&](const auto& b, bool valid) SG_INLINE {
-    bfp::blk_reverse(b, a, e0 + min(b.lane, envs - 1), valid);
-  });
+  bfp::Blk<bfp::BfpAlg, E> b;
+  b.init(model, smem, envs, true);
+  bfp::blk_reverse(b, model, smem, a, e0, e0 + min(b.el, envs - 1));
 }
 
+// The inputs of a vector-Jacobian product, the third among them at item x and the adjoint at item
+// bar: all of them, as results may lie where the arguments do.
+template <int E>
+__device__ __forceinline__ void vjp_load(const bfp::Blk<bfp::BfpAlg, E>& b, const VjpArgs& a, int x, int bar,
+                                         int64_t e) {
+  b.clear_notes(0);
+  __syncthreads();
+#pragma unroll 1
+  for (int c = b.slot; c < b.nq; c += b.slots) bfp::blk_in(b, c, ldv(a.q, e, c));
+#pragma unroll 1
+  for (int c = b.slot; c < b.nv; c += b.slots) {
+    bfp::blk_in(b, b.nq + c, ldv(a.qd, e, c));
+    bfp::blk_in(b, x + c, ldv(a.x, e, c));
+    b.set_in(bar + c, ldv(a.bar, e, c));
+  }
+  __syncthreads();
+}
 // Vector-Jacobian product of RNEA.
 template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_rnea_vjp_kernel(const DModel* __restrict__ model,
@@ -386,28 +481,22 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_rnea_vjp_kernel(cons
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, true, envs, [&](const auto& b, bool valid) SG_INLINE {
-    const int64_t e = e0 + min(b.lane, envs - 1);
-#pragma unroll 1
-    for (int c = b.slot; c < b.nq; c += b.slots) bfp::blk_in(b, c, ldv(a.q, e, c));
-#pragma unroll 1
-    for (int c = b.slot; c < b.nv; c += b.slots) {
-      bfp::blk_in(b, b.nq + c, ldv(a.qd, e, c));
-      bfp::blk_in(b, b.nq + b.nv + c, ldv(a.x, e, c));
-    }
-    __syncthreads();
-    bfp::blk_check_quaternion(b);
-    if (b.col >= 0) {
-      const double v = ldv(a.bar, e, b.ext[b.col]);
-      if (!bfp::bfp_fits(v)) b.refuse();
-      b.setD(b.L.b + b.nv + b.col, v);
-    }
-    __syncthreads();
-    bfp::blk_rnea_adjoint(b, [&](int c, int which, double v) SG_INLINE {
-      const Arr& o = which == 0 ? a.o1 : which == 1 ? a.o2 : a.o3;
-      if (valid && o.p && !bfp::blk_refused(b)) stv(o, e, b.ext[c], v);
-    });
-  });
+  blk_run<E>(
+      model, smem, true, envs, bfp::kLost,
+      [&](const auto& b) SG_INLINE { vjp_load(b, a, b.nq + b.nv, b.nq + 2 * b.nv, e0 + min(b.el, envs - 1)); },
+      [&](const auto& b) SG_INLINE {
+        const int64_t e = e0 + b.el;
+        if (b.col >= 0) {
+          const double v = b.tau(b.ext[b.col]);  // the adjoint
+          if (!bfp::bfp_fits(v)) b.refuse();
+          b.setD(b.L.b + b.nv + b.col, v);
+        }
+        __syncthreads();
+        bfp::blk_rnea_adjoint(b, [&](int c, int which, double v) SG_INLINE {
+          const Arr& o = which == 0 ? a.o1 : which == 1 ? a.o2 : a.o3;
+          if (b.valid && o.p) stv(o, e, b.ext[c], v);
+        });
+      });
 }
 // Vector-Jacobian product of forward dynamics.
 template <int E>
@@ -416,42 +505,35 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_aba_vjp_kernel(const
   extern __shared__ __align__(16) long long smem[];
   const int64_t e0 = int64_t(blockIdx.x) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
-  blk_run<E>(model, smem, true, envs, [&](const auto& b, bool valid) SG_INLINE {
-    const int64_t e = e0 + min(b.lane, envs - 1);
-    const int nv = b.nv;
+  blk_run<E>(
+      model, smem, true, envs, bfp::kLost,
+      [&](const auto& b) SG_INLINE { vjp_load(b, a, b.nq + 2 * b.nv, b.nq + 3 * b.nv, e0 + min(b.el, envs - 1)); },
+      [&](const auto& b) SG_INLINE {
+        const int64_t e = e0 + b.el;
+        const int nv = b.nv;
+        bfp::blk_forward_dynamics(b);
+        const int c = b.col, x = c >= 0 ? b.ext[c] : 0;
+        // qdd joins the inputs; the factor moves to Y's items; the right-hand side becomes the adjoint
+        if (c >= 0) {
+          const int i = b.row_start[c] + b.depth[c];
+          bfp::blk_in(b, b.nq + nv + x, b.D(b.L.b + nv + c));
+          b.setD(b.L.Y + i, bfp::blk_inverse_pivot(b, c));
+        }
 #pragma unroll 1
-    for (int c = b.slot; c < b.nq; c += b.slots) bfp::blk_in(b, c, ldv(a.q, e, c));
-#pragma unroll 1
-    for (int c = b.slot; c < nv; c += b.slots) {
-      bfp::blk_in(b, b.nq + c, ldv(a.qd, e, c));
-      bfp::blk_in(b, b.nq + 2 * nv + c, ldv(a.x, e, c));
-    }
-    __syncthreads();
-    bfp::blk_check_quaternion(b);
-    bfp::blk_forward_dynamics(b);
-    const int c = b.col, x = c >= 0 ? b.ext[c] : 0;
-    // qdd joins the inputs; the factor moves to Y's items; the right-hand side becomes the adjoint
-    double bar = 0.0;
-    if (c >= 0) {
-      const int i = b.row_start[c] + b.depth[c];
-      bfp::blk_in(b, b.nq + nv + x, b.D(b.L.b + nv + c));
-      bar = ldv(a.bar, e, x);
-      b.setD(b.L.Y + i, bfp::blk_inverse_pivot(b, c));
-    }
-#pragma unroll 1
-    for (int i = b.slot; i < b.npairs; i += b.slots)
-      if (b.pair_row[i] != b.pair_col[i]) b.setD(b.L.Y + i, b.D(b.L.S + i));
-    if (c >= 0) b.setD(b.L.b + c, bar);
-    __syncthreads();
-    bfp::blk_factor_solve(b);
-    const double lam = c >= 0 ? b.D(b.L.b + nv + c) : 0.0;
-    if (!bfp::bfp_fits(lam)) b.refuse();
-    bfp::blk_rnea_adjoint(b, [&](int col, int which, double v) SG_INLINE {
-      const Arr& o = which == 0 ? a.o1 : a.o2;
-      if (which < 2 && valid && o.p && !bfp::blk_refused(b)) stv(o, e, b.ext[col], -v);
-    });
-    if (c >= 0 && valid && a.o3.p && !bfp::blk_refused(b)) stv(a.o3, e, x, lam);
-  });
+        for (int i = b.slot; i < b.npairs; i += b.slots)
+          if (b.pair_row[i] != b.pair_col[i]) b.setD(b.L.Y + i, b.D(b.L.S + i));
+        if (c >= 0) b.setD(b.L.b + c, b.in(b.nq + 3 * nv + x));
+        __syncthreads();
+        bfp::blk_factor_solve(b);
+        const double lam = c >= 0 ? b.D(b.L.b + nv + c) : 0.0;
+        if (!bfp::bfp_fits(lam)) b.refuse();
+        bfp::blk_poses(b);
+        bfp::blk_rnea_adjoint(b, [&](int col, int which, double v) SG_INLINE {
+          const Arr& o = which == 0 ? a.o1 : a.o2;
+          if (which < 2 && b.valid && o.p) stv(o, e, b.ext[col], -v);
+        });
+        if (c >= 0 && b.valid && a.o3.p) stv(a.o3, e, x, lam);
+      });
 }
 #endif
 
