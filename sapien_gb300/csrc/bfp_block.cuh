@@ -1025,16 +1025,6 @@ __global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_passive_kernel(const 
         }
       });
 }
-
-// Launches a kernel with `smem` bytes of dynamic shared memory.
-template <class... P, class... Q>
-cudaError_t launch_block(void (*kernel)(P...), dim3 blocks, unsigned threads, size_t smem, cudaStream_t s,
-                         const Q&... args) {
-  if (smem > 48 * 1024)
-    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))) return e;
-  kernel<<<blocks, threads, smem, s>>>(args...);
-  return cudaGetLastError();
-}
 #endif
 
 }  // namespace sgdyn

@@ -4,8 +4,26 @@
 
 #include <map>
 #include <mutex>
+#include <set>
+#include <utility>
 
 namespace sgdyn {
+
+cudaError_t allow_shared(const void* kernel) {
+  static std::mutex mu;
+  static std::set<std::pair<const void*, int>> done;
+  int dev = 0, most = 0;
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kernel, dev})) return cudaSuccess;
+  cudaFuncAttributes own;
+  cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&own, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - int(own.sharedSizeBytes));
+  if (e == cudaSuccess) done.insert({kernel, dev});
+  return e;
+}
 
 namespace {
 int multiprocessors() {

@@ -182,9 +182,7 @@ cudaError_t launch_hetero_bucket(int ops, const HeteroArgs& a, dim3 grid, dim3 b
   switch (ops) {
 #define SG_CASE(O)                                                                                            \
   case O:                                                                                                     \
-    if (smem > 48 * 1024 &&                                                                                   \
-        cudaFuncSetAttribute(hetero_kernel<MAXJ, O>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != \
-            cudaSuccess)                                                                                      \
+    if (smem > 48 * 1024 && allow_shared(reinterpret_cast<const void*>(&hetero_kernel<MAXJ, O>)) != cudaSuccess) \
       return cudaErrorInvalidValue;                                                                           \
     hetero_kernel<MAXJ, O><<<grid, block, smem, s>>>(a);                                                      \
     break;

@@ -138,6 +138,10 @@ cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const S
 // Whether a process-wide setting of the FP64 sweeps (step splitting, forward-dynamics method) is
 // other than automatic: they then run.
 bool fp64_forced();
+// Lets a kernel be launched with all the shared memory a block can have on the current device. Once
+// per kernel and device, and never lowered: the limit is the kernel's, not a launch's, and other
+// threads' launches of the kernel with other models go by it.
+cudaError_t allow_shared(const void* kernel);
 // Whether launch_bfp_step can hold the model.
 bool bfp_step_fits(const BfpTree& t);
 cudaError_t launch_bfp_passive(const DModel* dm, const BfpTree& t, const PassiveArgs& a, cudaStream_t s);
