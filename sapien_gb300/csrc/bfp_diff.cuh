@@ -440,11 +440,13 @@ template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_replay_kernel(const DModel* __restrict__ model,
                                                                         const RolloutArgs a) {
   extern __shared__ __align__(16) long long smem[];
-  const int64_t e0 = int64_t(blockIdx.x) * E;
+  // segment after segment in one grid dimension: there may be more of them than the others hold
+  const unsigned per_segment = unsigned((a.n + E - 1) / E), g = blockIdx.x / per_segment;
+  const int64_t e0 = int64_t(blockIdx.x - g * per_segment) * E;
   const int envs = a.n - e0 < E ? int(a.n - e0) : E;
   bfp::Blk<bfp::BfpAlg, E> b;
   b.init(model, smem, envs);
-  bfp::blk_replay(b, model, smem, a, int(blockIdx.y), e0, e0 + min(b.el, envs - 1));
+  bfp::blk_replay(b, model, smem, a, int(g), e0, e0 + min(b.el, envs - 1));
 }
 template <int E>
 __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_reverse_kernel(const DModel* __restrict__ model,

@@ -8,8 +8,7 @@ cudaError_t launch_bfp_diff_e8(BfpDiff what, const DModel* dm, const RolloutArgs
                                 const BlkShape& b, cudaStream_t s) {
   switch (what) {
     case BfpDiff::rollout: return launch_block(bfp_rollout_kernel<8>, b.blocks, b.threads, b.smem, s, dm, *r);
-    case BfpDiff::replay:
-      return launch_block(bfp_replay_kernel<8>, dim3(b.blocks, unsigned(r->s_cnt)), b.threads, b.smem, s, dm, *r);
+    case BfpDiff::replay: return launch_block(bfp_replay_kernel<8>, b.blocks, b.threads, b.smem, s, dm, *r);
     case BfpDiff::reverse: return launch_block(bfp_reverse_kernel<8>, b.blocks, b.threads, b.smem, s, dm, *r);
     case BfpDiff::rnea_vjp: return launch_block(bfp_rnea_vjp_kernel<8>, b.blocks, b.threads, b.smem, s, dm, *v);
     case BfpDiff::aba_vjp: return launch_block(bfp_aba_vjp_kernel<8>, b.blocks, b.threads, b.smem, s, dm, *v);

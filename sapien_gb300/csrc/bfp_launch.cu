@@ -115,9 +115,8 @@ cudaError_t launch_bfp_diff(BfpDiff what, const DModel* dm, const BfpTree& t, co
   // fit or neither is used
   if (blk_shape(t, true, n).envs == 0) return cudaErrorNotSupported;
   const bool adjoint = what == BfpDiff::reverse || what == BfpDiff::rnea_vjp || what == BfpDiff::aba_vjp;
-  const BlkShape shape = blk_shape(t, adjoint, what == BfpDiff::replay ? n * r->s_cnt : n);
-  BlkShape b = shape;
-  b.blocks = unsigned((n + b.envs - 1) / b.envs);
+  BlkShape b = blk_shape(t, adjoint, what == BfpDiff::replay ? n * r->s_cnt : n);
+  b.blocks = unsigned((n + b.envs - 1) / b.envs) * unsigned(what == BfpDiff::replay ? r->s_cnt : 1);
   switch (b.envs) {
     case 4: return launch_bfp_diff_e4(what, dm, r, v, b, s);
     case 8: return launch_bfp_diff_e8(what, dm, r, v, b, s);
