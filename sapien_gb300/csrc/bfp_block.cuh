@@ -671,6 +671,7 @@ __device__ __forceinline__ void blk_mass_matrix(const Blk<A, E, EI>& b, bool for
     if (for_output) b.setD(b.L.Y + i, A::get(diag));
   }
   if (for_solve) __syncthreads();
+  bool beyond = false;
 #pragma unroll 1
   for (int i = b.slot; i < b.npairs; i += b.slots) {
     const int pa = b.pair_row[i], pc = b.pair_col[i];
@@ -679,6 +680,8 @@ __device__ __forceinline__ void blk_mass_matrix(const Blk<A, E, EI>& b, bool for
     if (for_solve) {
       if constexpr (A::kFixed) {
         const int k = v.e + 60 - b.X(b.L.xs + pa) - b.X(b.L.xs + pc);
+        // (more than 2 sqrt(M_aa M_cc): not positive definite, and it may not fit the word)
+        beyond = beyond || (v.m != 0 && k - clz32(abs_hi(v.m)) > -3);
         b.W(b.L.A + i) = k >= 0 ? shl(v.m, k) : shr(v.m, -k);
       } else {
         b.setD(b.L.A + i, v);
@@ -686,6 +689,7 @@ __device__ __forceinline__ void blk_mass_matrix(const Blk<A, E, EI>& b, bool for
     }
     if (for_output) b.setD(b.L.Y + i, A::get(v));
   }
+  if (beyond) b.refuse();
   __syncthreads();
 }
 
@@ -714,12 +718,14 @@ __device__ __forceinline__ void blk_back(const Blk<A, E, EI>& b);
 // Then L x = D^-1 y by levels, one product per column and level. M is in A: scaled fixed point
 // (M_ac = h_ac 2^(s_a + s_c - 60) with |h| <= 2^60, the scales from the diagonal: a positive
 // definite matrix has |M_ac| <= sqrt(M_aa M_cc), and so have the matrices that elimination
-// leaves; with D 4^x in [1/4, 1] every h_ac 2^x and f = h_ac 2^x / (D 4^x) stay below 1 and 2,
-// L_ac = f 2^(x_a + s_c - s_a)), or FP64.
+// leaves; with D 4^x in [1/4, 1] every h_ac 2^x and f = h_ac 2^x / (D 4^x) stay below 1 and 4,
+// L_ac = f 2^(x_a + s_c - s_a)), or FP64. Inertias that no body has can give another matrix: the
+// environment refuses with the first h_ac 2^x above 1.
 template <class A, int E, int EI>
 __device__ __forceinline__ void blk_solve(const Blk<A, E, EI>& b) {
   const int nv = b.nv, col = b.col;
   const int row = col >= 0 ? b.L.A + b.row_start[col] : 0, dr = col >= 0 ? b.depth[col] : nv;
+  bool beyond = false;
   if (dr == b.col_levels - 1) blk_pivot(b, col, row + dr);
   __syncthreads();
 #pragma unroll 1
@@ -733,7 +739,9 @@ __device__ __forceinline__ void blk_solve(const Blk<A, E, EI>& b) {
         const double ba = b.D(b.L.b + a);
         if constexpr (A::kFixed) {
           const int xa = b.X(b.L.xs + nv + a);
-          const Half4 f = split4(mul60(split4(shl(b.W(h0 + dr), xa)), split4(b.W(h0 + da))));
+          const i64 h = b.W(h0 + dr);
+          beyond = beyond || abs_hi(h) > (1u << 28 >> xa) + 1;
+          const Half4 f = split4(mul60(split4(shl(h, xa)), split4(b.W(h0 + da))));
 #pragma unroll 1
           for (int d = 0; d <= dr; d++) b.W(row + d) -= shl(mul60(f, split4(shl(b.W(h0 + d), xa))), 2);
           const double l = to_double(shl(i64(f.h), 32) + f.l, xa - 58 + b.X(b.L.xs + col) - b.X(b.L.xs + a));
@@ -754,6 +762,7 @@ __device__ __forceinline__ void blk_solve(const Blk<A, E, EI>& b) {
       else dinv = b.D(row + dr);
       b.setD(b.L.b + nv + col, b.D(b.L.b + col) * dinv);
     }
+    if (da == 0 && beyond) b.refuse();
     __syncthreads();
   }
   blk_back(b);

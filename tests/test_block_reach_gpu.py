@@ -1,10 +1,12 @@
 """Calls at the edges of the block sweeps' reach."""
 import ctypes
 
+import numpy as np
 import pytest
 
+from sapien_gb300 import PinocchioModel
 from sapien_gb300 import _native as N
-from test_bfp_gpu import ROBOTS, cuda, pair
+from test_bfp_gpu import ROBOTS, cuda, fp64_route, host, pair, rel_per_env
 
 pytestmark = pytest.mark.gpu
 
@@ -29,3 +31,46 @@ def test_more_checkpoint_segments_than_a_grid_has_rows():
               for b in (1 << 30, 5000 * need.value)]
     for a, b in zip(*groups):
         assert torch.isfinite(a).all() and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("ixz", [0.02, 0.05, 0.1, 0.503, 1.002, -2.01, 30.0])
+def test_mass_matrix_that_is_not_positive_definite(ixz):
+    """Products of inertia beyond the moments': M = [[a, h], [h, c]] with h^2 up to millions of times
+    a c, alone and below another joint. Forward dynamics and its product as in FP64."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    def body(name, xx, xz):
+        return (f'<link name="{name}"><inertial><mass value="1"/><origin xyz="0 0 0" rpy="0 0 0"/>'
+                f'<inertia ixx="{xx}" iyy="0.03" izz="0.01" ixy="0" ixz="{xz}" iyz="0"/></inertial></link>')
+
+    def joint(name, parent, child, axis):
+        return (f'<joint name="{name}" type="continuous"><origin xyz="0 0 0.1" rpy="0 0 0"/><axis xyz="{axis}"/>'
+                f'<parent link="{parent}"/><child link="{child}"/></joint>')
+
+    for axes in (["0 0 1", "1 0 0"], ["0 1 0", "0 0 1", "1 0 0"]):
+        names = [f"j{k}" for k in range(len(axes))]
+        links = [f"l{k}" for k in range(len(axes) + 1)]
+        pm = PinocchioModel("<robot name='r'>" + "".join(body(x, 0.01, ixz if x == links[-1] else 0) for x in links)
+                            + "".join(joint(names[k], links[k], links[k + 1], a) for k, a in enumerate(axes))
+                            + "</robot>", [0, 0, -9.81])
+        pm.set_joint_order(names)
+        pm.set_link_order(links)
+        rng = np.random.default_rng(1)
+        q = 0.3 * rng.normal(size=(9, len(axes)))
+        qd, tau = rng.normal(size=q.shape), rng.normal(size=q.shape)
+
+        def run():
+            out = [pm.step_batched(*cuda(q, qd, 0 * q, tau), ops=o)["qacc"] for o in (N.OP_ALL, N.OP_FORWARD_DYNAMICS)]
+            return [x.cpu().numpy() for x in out]
+
+        mine = run()
+        with fp64_route():
+            want = run()
+        for a, b in zip(mine, want):
+            assert rel_per_env(a, b) <= 1e-9
+        w = torch.ones(q.shape, dtype=torch.float64, device="cuda")
+        tb = AD.forward_dynamics_vjp(pm, *cuda(q, qd, tau), w)[2].cpu().numpy()
+        M = host(pm.step_batched(*cuda(q), ops=N.OP_MASS_MATRIX))["mass_matrix"].reshape(len(q), len(axes), len(axes))
+        assert rel_per_env(tb, np.linalg.solve(M, np.ones(q.shape)[..., None])[..., 0]) <= 1e-9
