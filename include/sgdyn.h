@@ -182,6 +182,10 @@ int sgdyn_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const 
  * in FP64. (Addition.) */
 int sgdyn_step_split(int mode, int* mode_out);
 
+/* Whether the block sweep serves the model as the settings stand (addition): 1 or 0 to *serves. 0:
+ * one of its constants is out of range, its tree does not fit, or a setting asks for FP64. */
+int sgdyn_model_block_sweep(const sgdyn_model* m, int* serves);
+
 /* Lanes per environment for the single-model fused sweep and single-op entry points
  * (addition): 0 = automatic (default), 1, 2, 4 or 8. With L > 1 a team of L lanes shares an
  * environment: the joints near the root run on every lane and the subtrees off them on one

@@ -43,6 +43,7 @@ EXPORTED = (
     "sgdyn_model_body_name",
     "sgdyn_model_upload",
     "sgdyn_model_table",
+    "sgdyn_model_block_sweep",
     "sgdyn_compute_forward_kinematics",
     "sgdyn_compute_full_jacobian",
     "sgdyn_compute_link_jacobian",
@@ -124,6 +125,7 @@ def load():
     L.sgdyn_model_body_name.argtypes = [vp, i32, P(ctypes.c_char_p)]
     L.sgdyn_model_upload.argtypes = [vp]
     L.sgdyn_model_table.argtypes = [vp, P(vp), P(i64)]
+    L.sgdyn_model_block_sweep.argtypes = [vp, P(i32)]
     L.sgdyn_compute_forward_kinematics.argtypes = [vp, i64, vp, vp, i32, vp]
     L.sgdyn_compute_full_jacobian.argtypes = [vp, i64, vp, vp, i32, vp]
     L.sgdyn_compute_link_jacobian.argtypes = [vp, i64, i32, i32, vp, vp, i32, vp]

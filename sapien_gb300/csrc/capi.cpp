@@ -189,6 +189,9 @@ int choose_lanes(Model& M, int64_t n) {
   return best;
 }
 
+// Whether a model's calls go to the block sweeps, as far as settings and its constants say.
+bool block_sweep(const Model& M) { return M.bfp_ok() && M.lanes == 0 && !fp64_forced(); }
+
 BfpTree bfp_tree(const Model& M) { return {M.njoints(), M.nv(), M.nq_ext(), M.btree().npairs, M.btree().nints}; }
 
 int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const double* qd, const double* qdd,
@@ -232,8 +235,7 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
   // With every setting automatic: the block-floating-point sweep, one launch for any op set and
   // batch size (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings
   // (lanes, split, forward-dynamics route) and what that sweep cannot hold.
-  if (Mo.bfp_ok() && Mo.lanes == 0 && !fp64_forced() &&
-      !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
+  if (block_sweep(Mo) && !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
     const cudaError_t e = launch_bfp_step(dm, bfp_tree(Mo), ops, a, s);
     if (e == cudaSuccess) return SGDYN_OK;
     if (e != cudaErrorNotSupported)
@@ -453,6 +455,14 @@ int sgdyn_model_table(const sgdyn_model* m, const void** data, int64_t* bytes) {
   if (!m || !data || !bytes) return fail(SGDYN_ERR_NULL, "null argument");
   *data = m->impl->host_table().data();
   *bytes = int64_t(m->impl->host_table().size());
+  return SGDYN_OK;
+}
+
+int sgdyn_model_block_sweep(const sgdyn_model* m, int* serves) {
+  if (int rc = check_model(m)) return rc;
+  if (!serves) return fail(SGDYN_ERR_NULL, "null argument");
+  const Model& M = *m->impl;
+  *serves = block_sweep(M) && bfp_step_fits(bfp_tree(M)) ? 1 : 0;
   return SGDYN_OK;
 }
 

@@ -634,10 +634,15 @@ int to_block(const long double* v, int n, long long* out) {
   for (int k = 0; k < n; k++) out[k] = mantissa(v[k], e);
   return e;
 }
+// Whether a block's largest entry is 0 or within 2^+-100. The others need no lower bound: below
+// 2^-61 of the largest they become 0, such as the residues of rpy="pi 0 pi/2" in a rotation.
 bool in_range(const double* v, int n) {
-  for (int k = 0; k < n; k++)
-    if (!(v[k] == 0 || (std::fabs(v[k]) > 0x1p-100 && std::fabs(v[k]) < 0x1p100))) return false;
-  return true;
+  double most = 0;
+  for (int k = 0; k < n; k++) {
+    if (!(std::fabs(v[k]) < 0x1p100)) return false;
+    most = std::max(most, std::fabs(v[k]));
+  }
+  return most == 0 || most > 0x1p-100;
 }
 }  // namespace
 

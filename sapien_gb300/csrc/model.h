@@ -104,8 +104,8 @@ class Model {
   // Host copy of the packed table (for tests and for the heterogeneous packer).
   const std::vector<unsigned char>& host_table() const { return table_; }
   // The block-floating-point constants (BJoint per joint, then BLink per link), and whether
-  // every constant of the model is zero or within 2^+-100, as those sweeps need. After them the
-  // BTree and its ints.
+  // the largest entry of every constant vector and matrix is zero or within 2^+-100, as those
+  // sweeps need. After them the BTree and its ints.
   const std::vector<unsigned char>& bfp_table() const { return bfp_; }
   bool bfp_ok() const { return bfp_ok_; }
   const BTree& btree() const { return btree_; }

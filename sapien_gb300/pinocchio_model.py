@@ -231,6 +231,14 @@ class PinocchioModel:
         lanes share one environment of a wide tree, which pays off for small batches."""
         N.check(N.load().sgdyn_model_set_lanes(self._h, int(lanes)))
 
+    @property
+    def block_sweep(self):
+        """Whether the batched calls take the block sweep (block floating point) as the settings
+        stand, not the FP64 kernels: the model's constants are in its range and its tree fits."""
+        v = ctypes.c_int()
+        N.check(N.load().sgdyn_model_block_sweep(self._h, ctypes.byref(v)))
+        return bool(v.value)
+
     def table_bytes(self):
         """Host copy of the packed kernel tables (see csrc/device_model.h)."""
         L = N.load()

@@ -74,3 +74,21 @@ def test_mass_matrix_that_is_not_positive_definite(ixz):
         tb = AD.forward_dynamics_vjp(pm, *cuda(q, qd, tau), w)[2].cpu().numpy()
         M = host(pm.step_batched(*cuda(q), ops=N.OP_MASS_MATRIX))["mass_matrix"].reshape(len(q), len(axes), len(axes))
         assert rel_per_env(tb, np.linalg.solve(M, np.ones(q.shape)[..., None])[..., 0]) <= 1e-9
+
+
+def test_right_angles_in_the_placements():
+    """rpy="pi 0 pi/2" leaves entries of 1e-17 and 1e-32 in a rotation: the block sweep takes the model
+    and matches the FP64 kernels."""
+    from test_block_sweep_range import arm
+
+    pm = arm("3.141592653589793 0 1.5707963267948966")
+    assert pm.block_sweep
+    pm.set_joint_order(["j", "k"])
+    pm.set_link_order(["base", "a", "b"])
+    ins = cuda(*np.random.default_rng(3).normal(size=(4, 37, 2)))
+    got = host(pm.step_batched(*ins))
+    with fp64_route():
+        assert not pm.block_sweep
+        want = host(pm.step_batched(*ins))
+    for k in got:
+        assert rel_per_env(got[k], want[k]) <= 1e-12, k
