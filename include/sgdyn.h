@@ -176,10 +176,12 @@ int sgdyn_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const 
  * Automatic, with lanes per environment and forward-dynamics method automatic too: one launch of
  * the block sweep for any set of ops (block floating point, a block of threads per group of
  * environments), for every model with constants that are 0 or within 2^+-100 and a tree that
- * fits a block's shared memory. Other models, and any other value of these settings: the FP64
- * kernels, as two launches while the batch gives fewer than two warps per FP64 scheduler and
- * `stream` is not being captured. Modes 0 and 1 also keep mixed batches and inverse kinematics
- * in FP64. (Addition.) */
+ * fits a block's shared memory; rollouts, vector-Jacobian products and passive forces likewise.
+ * Other models, and any other value of these settings: the FP64 kernels, a five-op step as two
+ * launches while the batch gives fewer than two warps per FP64 scheduler and `stream` is not being
+ * captured. Modes 0 and 1, and a forward-dynamics method, also keep mixed batches and inverse
+ * kinematics in FP64; lanes per environment are a model's own and do not reach these two.
+ * (Addition.) */
 int sgdyn_step_split(int mode, int* mode_out);
 
 /* Whether the block sweep serves the model as the settings stand (addition): 1 or 0 to *serves. 0:

@@ -153,7 +153,8 @@ bool fp64_forced() {
   fd_method(-1, &fd);
   return g_split_mode.load() != 2 || fd != 0;
 }
-
+bool block_sweep(const Model& M) { return M.bfp_ok() && M.lanes == 0 && !fp64_forced(); }
+BfpTree bfp_tree(const Model& M) { return {M.njoints(), M.nv(), M.nq_ext(), M.btree().npairs, M.btree().nints}; }
 
 // Lanes per environment of the rollout kernels for this model and batch (1 or 3).
 int rollout_lanes_for(const Model& M, int64_t n) { return rollout_lanes(M, n); }
@@ -188,11 +189,6 @@ int choose_lanes(Model& M, int64_t n) {
   }
   return best;
 }
-
-// Whether a model's calls go to the block sweeps, as far as settings and its constants say.
-bool block_sweep(const Model& M) { return M.bfp_ok() && M.lanes == 0 && !fp64_forced(); }
-
-BfpTree bfp_tree(const Model& M) { return {M.njoints(), M.nv(), M.nq_ext(), M.btree().npairs, M.btree().nints}; }
 
 int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const double* qd, const double* qdd,
              const double* tau, double* poses, double* J, double* M, double* tau_out, double* qdd_out, int layout,
@@ -735,7 +731,7 @@ int sgdyn_compute_inverse_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(qdd_bar, n, nv, layout);
-    if (Mo.bfp_ok()) {
+    if (block_sweep(Mo)) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::rnea_vjp, dm, bfp_tree(Mo), nullptr, &a,
                                             static_cast<cudaStream_t>(stream));
       if (e != cudaErrorNotSupported) return launch_status(e);
@@ -777,7 +773,7 @@ int sgdyn_compute_forward_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     // 24576: 800 against 651; 35-DoF humanoid, 32768: 2325 against 1654; 9-DoF arm, 4.9 pairs,
     // 131072: 1371 against 1637).
     const bool long_chains = Mo.btree().npairs > 6 * Mo.nv();
-    if (Mo.bfp_ok() && !(long_chains && n > 32 * int64_t(device_schedulers()))) {
+    if (block_sweep(Mo) && !(long_chains && n > 32 * int64_t(device_schedulers()))) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::aba_vjp, dm, bfp_tree(Mo), nullptr, &a,
                                             static_cast<cudaStream_t>(stream));
       if (e != cudaErrorNotSupported) return launch_status(e);
@@ -910,7 +906,7 @@ int sgdyn_rollout_forward(const sgdyn_model* m, int64_t n, int T, double dt, con
     a.qT = qT; a.qdT = qdT; a.q_ckpt = q_ckpt; a.qd_ckpt = qd_ckpt;
     std::string why;
     const auto st = static_cast<cudaStream_t>(stream);
-    if (Mo.bfp_ok() && g_rollout_lanes.load() == 0) {
+    if (block_sweep(Mo) && g_rollout_lanes.load() == 0) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::rollout, dm, bfp_tree(Mo), &a, nullptr, st);
       if (e != cudaErrorNotSupported) return launch_status(e);
     }
@@ -1028,7 +1024,7 @@ int sgdyn_rollout_backward(const sgdyn_model* m, int64_t n, int T, double dt, in
     a.q0_bar = q0_bar; a.qd0_bar = qd0_bar; a.tau_bar = tau_bar; a.scratch = scratch;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nj = Mo.njoints();
-    if (Mo.bfp_ok() && g_rollout_lanes.load() == 0 && T > 0) {
+    if (block_sweep(Mo) && g_rollout_lanes.load() == 0 && T > 0) {
       // its records are smaller than the intermediates the scratch is sized for
       const BfpTree tree = bfp_tree(Mo);
       const int64_t seg = bfp_record_doubles(tree) * checkpoint_every * n;

@@ -433,7 +433,7 @@ int sgdyn_batch_create(const sgdyn_model* const* models, int nmodels, const int*
     const auto& c = m->impl->bfp_table();
     packed.insert(packed.end(), c.begin(), c.end());
     const Model& M = *m->impl;
-    b->trees.push_back({M.njoints(), M.nv(), M.nq_ext(), M.btree().npairs, M.btree().nints});
+    b->trees.push_back(bfp_tree(M));
     b->bfp = b->bfp && M.bfp_ok() && bfp_step_fits(b->trees.back());
     while (packed.size() % 256) packed.push_back(0);
   }

@@ -138,6 +138,11 @@ cudaError_t launch_bfp_step(const DModel* dm, const BfpTree& t, int ops, const S
 // Whether a process-wide setting of the FP64 sweeps (step splitting, forward-dynamics method) is
 // other than automatic: they then run.
 bool fp64_forced();
+// Whether a model's calls go to the block sweeps, as far as its constants and the settings say: these,
+// and lanes per environment of the model's own.
+class Model;
+bool block_sweep(const Model& M);
+BfpTree bfp_tree(const Model& M);
 // Lets a kernel be launched with all the shared memory a block can have on the current device. Once
 // per kernel and device, and never lowered: the limit is the kernel's, not a launch's, and other
 // threads' launches of the kernel with other models go by it.

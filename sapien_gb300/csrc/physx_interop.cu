@@ -92,10 +92,9 @@ extern "C" int sgdyn_compute_passive_force_f32(const sgdyn_model* m, int64_t n, 
   const unsigned blocks = unsigned((n + 31) / 32);
   auto s = static_cast<cudaStream_t>(stream);
   // block floating point (bfp_block.cuh): 4096 9-DoF arms 102 -> 29 us; the FP64 kernel below
-  // for models it cannot hold
-  if (Mo.bfp_ok()) {
-    const BfpTree t{Mo.njoints(), Mo.nv(), Mo.nq_ext(), Mo.btree().npairs, Mo.btree().nints};
-    const cudaError_t e = launch_bfp_passive(dm, t, a, s);
+  // for models it cannot hold and settings that ask for FP64
+  if (block_sweep(Mo)) {
+    const cudaError_t e = launch_bfp_passive(dm, bfp_tree(Mo), a, s);
     if (e == cudaSuccess) return SGDYN_OK;
     if (e != cudaErrorNotSupported)
       return set_last_error(SGDYN_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString(e));
