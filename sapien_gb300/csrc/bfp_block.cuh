@@ -292,13 +292,15 @@ struct Blk {
     p = ti[t.parent + j];
     lv = ti[t.level + j];
   }
-  // The first `envs` of the block's environments.
+  // The first `envs` of the block's environments; the tree and the first notes are there after it.
   __device__ __forceinline__ void init(const DModel* model, long long* smem, int envs, bool adjoint = false) {
     setup(model, smem, adjoint, false);
     el = lane;
     count = envs;
     valid = lane < envs;
     set = 0;
+    clear_notes(0);
+    __syncthreads();
   }
   // Those in `which` (E = 0), packed side by side so that a few of them take a few warps' issue.
   // Lanes beyond them repeat the last one and share its inputs: only valid ones may change these.
@@ -814,8 +816,6 @@ __device__ __forceinline__ void blk_in(const Blk<A, E, EI>& b, int at, double v)
 // Reads the environment's inputs; whether they suit BfpAlg goes to its notes.
 template <class A, int E, int EI>
 __device__ __forceinline__ void blk_load(const Blk<A, E, EI>& b, int ops, const StepArgs& args, int64_t e) {
-  b.clear_notes(0);
-  __syncthreads();
 #pragma unroll 1
   for (int c = b.slot; c < b.nq; c += b.slots) blk_in(b, c, ldv(args.q, e, c));
 #pragma unroll 1
@@ -1014,8 +1014,6 @@ __global__ void __launch_bounds__(bfp::kBlkMaxThreads) bfp_passive_kernel(const 
       model, smem, false, envs, bfp::kLostFloat,
       [&](auto& b) SG_INLINE {
         const int64_t e = e0 + min(b.el, envs - 1);
-        b.clear_notes(0);
-        __syncthreads();
         if (b.col >= 0) {  // one-DoF joints only: as many coordinates as columns
           bfp::blk_in(b, b.col, double(a.qpos[e * a.in_stride + b.col]));
           bfp::blk_in(b, b.nq + b.col, a.coriolis ? double(a.qvel[e * a.in_stride + b.col]) : 0.0);

@@ -94,8 +94,6 @@ template <int E, class R, class F>
 __device__ __forceinline__ void blk_steps(Blk<BfpAlg, E>& b, const DModel* model, long long* smem, const RolloutArgs& a,
                                           int64_t e, int t0, int t1, const R& record, const F& after) {
   const int nq = b.nq, nv = b.nv;
-  b.clear_notes(0);
-  b.set = 0;
   __syncthreads();
 #pragma unroll 1
   for (int t = t0; t < t1; t++) {
@@ -396,7 +394,6 @@ __device__ __forceinline__ void blk_reverse(Blk<BfpAlg, E>& b, const DModel* mod
     b.set_in(nq + 2 * nv + c, qin ? qin[e * nq + qx] : 0.0);
     b.set_in(nq + 3 * nv + c, qdin ? qdin[e * nv + x] : 0.0);
   }
-  b.clear_notes(0);
   __syncthreads();
 #pragma unroll 1
   for (int s = a.s_lo + a.s_cnt - 1; s >= a.s_lo; s--) {
@@ -464,8 +461,6 @@ __global__ void __launch_bounds__(bfp::kBlkDiffThreads) bfp_reverse_kernel(const
 template <int E>
 __device__ __forceinline__ void vjp_load(const bfp::Blk<bfp::BfpAlg, E>& b, const VjpArgs& a, int x, int bar,
                                          int64_t e) {
-  b.clear_notes(0);
-  __syncthreads();
 #pragma unroll 1
   for (int c = b.slot; c < b.nq; c += b.slots) bfp::blk_in(b, c, ldv(a.q, e, c));
 #pragma unroll 1

@@ -92,3 +92,29 @@ def test_right_angles_in_the_placements():
         want = host(pm.step_batched(*ins))
     for k in got:
         assert rel_per_env(got[k], want[k]) <= 1e-12, k
+
+
+@pytest.mark.parametrize("name,n", [("arm9", 2500), ("arm9", 5000), ("arm9", 9800), ("quadruped", 5000),
+                                    ("mixed", 9800)])
+def test_rollout_and_reverse_pass_in_blocks_of_every_size(name, n):
+    """Blocks of 8, 16 and 32 environments, a partly filled last one, two checkpoint segments: the
+    FP64 kernels' results."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    q, qd, _, tau = cuda(*robot.sample(n, seed=n))
+    taus = (0.1 * tau).unsqueeze(0).repeat(3, 1, 1).contiguous()
+    (bar,) = cuda(np.random.default_rng(4).normal(size=qd.shape))
+
+    def run():
+        qT, qdT, qc, qdc = AD.rollout_forward(pm, q, 0.1 * qd, taus, 1e-3, 2)
+        return [qT, qdT, *AD.rollout_backward(pm, qc, qdc, taus, 1e-3, 2, torch.ones_like(qT), bar)]
+
+    mine = run()
+    with fp64_route():
+        want = run()
+    for i, (a, b) in enumerate(zip(mine, want)):
+        assert rel_per_env(*(t.cpu().numpy().reshape(-1, t.shape[-1]) for t in (a, b))) <= 1e-8, i
