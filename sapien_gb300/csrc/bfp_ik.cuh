@@ -75,7 +75,12 @@ __device__ __forceinline__ double inverse_sqrt(double d) {
 }
 
 // One environment; false where it needs the FP64 kernel (an input out of range, a mask entry
-// that is not 0 or 1, a free flyer on the path, a normal matrix that is not positive definite).
+// that is not 0 or 1, a free flyer on the path, a normal matrix that is not positive definite; and
+// one whose steps or result are small as a whole: rotations are in steps of 2^-60 here, so a first
+// error of 1e-9 would be off by 1e-9 of itself, and the joints with it, where FP64 keeps it to its
+// last bits along the frames' axes. A first error below kIkSmall is below the usual tolerances and
+// then ends at once in FP64 too.)
+constexpr double kIkSmall = 1.0 / (1 << kSmall);
 template <int MAXJ>
 __device__ __forceinline__ bool ik_env(const DModel* __restrict__ model, const IkArgs& a, const int64_t e) {
   const DJoint* __restrict__ JT = model_joints(model);
@@ -202,7 +207,7 @@ __device__ __forceinline__ bool ik_env(const DModel* __restrict__ model, const I
       err.w = om;
     }
     const double nrm = sqrt(dot6(err, err));
-    if (!(nrm < 1e60)) return false;
+    if (!(nrm < 1e60) || (it == 0 && nrm < kIkSmall)) return false;
     if (nrm < minErr) {
       minErr = nrm;
       bestErr = err;
@@ -344,6 +349,10 @@ __device__ __forceinline__ bool ik_env(const DModel* __restrict__ model, const I
       }
     }
   }
+  double moved = 0.0;
+#pragma unroll 1
+  for (int i = 1; i < nj; i++) moved = fmax(moved, fabs(best[i]));
+  if (moved != 0.0 && moved < kIkSmall) return false;
 #pragma unroll 1
   for (int i = 1; i < nj; i++)
     stv(a.q_out, e, JT[i].qcol, JT[i].kind == JK_CONTINUOUS ? atan2(best[i], bestc[i]) : best[i]);
