@@ -259,20 +259,27 @@ def hetero_only(dev, which):
     args = (hb.pad_q([x[0] for x in ins]), hb.pad_v([x[1] for x in ins]), hb.pad_v([x[2] for x in ins]),
             hb.pad_v([x[3] for x in ins]))
     out = hb.alloc_outputs(OPS_DYNAMICS)
+    hb.set_fp64(True)  # what launch shapes and lanes are for
     hb.set_launch(2, 1, 0)
     hb.set_lanes([1, 1, 4])
     hb.step(*args, OPS_DYNAMICS, out)
     torch.cuda.synchronize()
     ms = _event_ms(torch, lambda: hb.step(*args, OPS_DYNAMICS, out), reps=3, warm=0)
-    return {"workload": f"{len(moe)} envs ({which}), RNEA+ABA+CRBA", "ms_per_step": ms, "launch_shape": [2, 1, 0],
-            "lanes_per_env": [1, 1, 4]}
+    return {"workload": f"{len(moe)} envs ({which}), RNEA+ABA+CRBA", "ms_per_step": ms, **_hetero_kernels(hb)}
+
+
+def _hetero_kernels(hb):
+    """What stepped a mixed batch: the block sweep, or the FP64 kernels as they were shaped."""
+    if hb.block_sweep:
+        return {"kernels": "block sweep, a launch per model"}
+    return {"kernels": "FP64", "launch_shape": list(hb.launch), "lanes_per_env": list(hb.lanes)}
 
 
 def secondary_workloads(dev, only_rollout=False):
     """The other workloads of the benchmark spec, timed with CUDA events on rank 0:
     differentiable rollout (9-DoF arm, 4096 envs, 200 steps, dt 1/500, q/qd checkpoints
     every 20 steps), heterogeneous batch (8192 mixed robots, RNEA + ABA + CRBA, CUDA-graph
-    replay, autotuned launch), batched CLIK (65536 targets, 100 iterations, damping 1e-3)
+    replay), batched CLIK (65536 targets, 100 iterations, damping 1e-3)
     and dense derivatives on the floating-base humanoid (8192 envs)."""
     import torch
 
@@ -311,24 +318,26 @@ def secondary_workloads(dev, only_rollout=False):
     hb = HeteroBatch(models, moe, device=dev)
     hq, hqd, hqdd, htau = (hb.pad_q([x[0] for x in ins]), hb.pad_v([x[1] for x in ins]),
                            hb.pad_v([x[2] for x in ins]), hb.pad_v([x[3] for x in ins]))
-    shape, _ = autotune.tune_batch(hb, hq, hqd, hqdd, htau, OPS_DYNAMICS)
+    # (launch shapes and lanes shape the FP64 kernels alone)
+    if not hb.block_sweep:
+        autotune.tune_batch(hb, hq, hqd, hqdd, htau, OPS_DYNAMICS)
     g = hb.capture(hq, hqd, hqdd, htau, steps=10)
     hms = _event_ms(torch, g.replay, reps=5, warm=1) / 10
     out["hetero"] = {"workload": "8192 envs: 50% 6-DoF arms, 30% 18-DoF quadrupeds, 20% 35-DoF humanoids; "
                                  "RNEA+ABA+CRBA; CUDA-graph replay of 10 steps",
-                     "env_steps_per_s": 8192 / (hms * 1e-3), "ms_per_step": hms, "launch_shape": list(shape),
-                     "lanes_per_env": list(hb.lanes)}
+                     "env_steps_per_s": 8192 / (hms * 1e-3), "ms_per_step": hms, **_hetero_kernels(hb)}
     out["hetero"].update(_hetero_parity(robots, moe, hb, g.outputs, ins))
     # a whole heterogeneous rollout (ABA + semi-implicit Euler, free flyers on SE(3)) as one graph,
-    # with the launch shape and lanes tuned for ABA alone
+    # in FP64 with the launch shape and lanes tuned for ABA alone
     rq, rqd, rtau = hq.clone(), hqd.clone(), 0.1 * htau
-    rshape, _ = autotune.tune_batch(hb, hq, hqd, hqdd, rtau, N.OP_FORWARD_DYNAMICS)
+    if not hb.block_sweep:
+        autotune.tune_batch(hb, hq, hqd, hqdd, rtau, N.OP_FORWARD_DYNAMICS)
     rg = hb.capture_rollout(rq, rqd, rtau, 1.0 / 500, 100)
     rms = _event_ms(torch, rg.replay, reps=3, warm=1) / 100
     out["hetero_rollout"] = {"workload": "same 8192-robot mix, 100 semi-implicit-Euler steps (ABA + integrate) "
                                          "captured as one CUDA graph, dt=1/500",
                              "env_steps_per_s": 8192 / (rms * 1e-3), "ms_per_step": rms,
-                             "launch_shape": list(rshape), "lanes_per_env": list(hb.lanes)}
+                             **_hetero_kernels(hb)}
     # parity: one replay (100 steps) from the initial state against the oracle's rollout
     rq.copy_(hq)
     rqd.copy_(hqd)

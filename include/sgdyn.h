@@ -298,6 +298,10 @@ int sgdyn_batch_set_launch(sgdyn_batch* b, int ctas_per_sm, int warps_per_cta, i
 /* (Launch shapes and lanes are those of the FP64 kernels: a batch whose models all fit the block
  * sweep takes one launch of it per model, see sgdyn_step_split.) */
 int sgdyn_batch_set_lanes(sgdyn_batch* b, const int* lanes_per_model);
+/* The kernels of one batch (addition): fp64 1 = the FP64 kernels, 0 = automatic (the default),
+ * -1 only reads. *fp64_out: the choice; *block_sweep: 1 when the block sweep serves the batch as
+ * all settings stand (either may be NULL). */
+int sgdyn_batch_route(sgdyn_batch* b, int fp64, int* fp64_out, int* block_sweep);
 int sgdyn_batch_step(sgdyn_batch* b, int ops, const double* q, const double* qd, const double* qdd, const double* tau,
                      double* link_poses, double* J, double* M, double* tau_out, double* qdd_out, void* stream);
 /* Semi-implicit Euler on the batch's padded rows, in place: qd += dt qdd, then q advanced

@@ -69,6 +69,7 @@ EXPORTED = (
     "sgdyn_batch_info",
     "sgdyn_batch_set_launch",
     "sgdyn_batch_set_lanes",
+    "sgdyn_batch_route",
     "sgdyn_batch_step",
     "sgdyn_batch_integrate",
     "sgdyn_batch_step_integrate",
@@ -158,6 +159,7 @@ def load():
     L.sgdyn_batch_info.argtypes = [vp, P(i64), P(i32), P(i32), P(i32)]
     L.sgdyn_batch_set_launch.argtypes = [vp, i32, i32, i32]
     L.sgdyn_batch_set_lanes.argtypes = [vp, P(i32)]
+    L.sgdyn_batch_route.argtypes = [vp, i32, P(i32), P(i32)]
     L.sgdyn_batch_step.argtypes = [vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]
     L.sgdyn_batch_integrate.argtypes = [vp, dbl, vp, vp, vp, vp]
     L.sgdyn_batch_step_integrate.argtypes = [vp, dbl, vp, vp, vp, vp, vp]

@@ -1,4 +1,8 @@
-"""Launch-shape and threads-per-environment autotuner.
+"""Launch-shape and threads-per-environment autotuner of the FP64 kernels.
+
+The settings are those of the FP64 kernels for heterogeneous batches, and these run while the
+tuner times them: also for a batch that the block sweep serves otherwise (`HeteroBatch.block_sweep`),
+whose steps they do not change.
 
 For a heterogeneous batch the tuner times, with CUDA events (median of a few launches
 after warm-up):
@@ -17,6 +21,7 @@ pays for the search once per tree mix.
 """
 from __future__ import annotations
 
+import contextlib
 import json
 import os
 import time
@@ -53,10 +58,20 @@ def _time(fn, reps=5):
     return float(np.median(ts))
 
 
+@contextlib.contextmanager
+def _fp64_kernels(batch):
+    was = batch.fp64
+    batch.set_fp64(True)
+    try:
+        yield
+    finally:
+        batch.set_fp64(was)
+
+
 def tune_batch(batch, q, qd, qdd, tau, ops, use_cache=True, candidates=None, lane_candidates=(1, 2, 4, 8)):
-    """Pick the fastest launch shape and lanes per environment for `batch` on these inputs,
-    apply them to the batch and return (shape, table); the lanes are in batch.lanes."""
-    key = f"{torch.cuda.get_device_name(batch.device)}|{batch_signature(batch, ops)}|lanes{tuple(lane_candidates)}"
+    """Pick the launch shape and lanes per environment with which the FP64 kernels step `batch` fastest
+    on these inputs, apply them to the batch and return (shape, table); the lanes are in batch.lanes."""
+    key = f"{torch.cuda.get_device_name(batch.device)}|{batch_signature(batch, ops)}|lanes{tuple(lane_candidates)}|fp64"
     path = _cache_path()
     cache = {}
     if use_cache and os.path.exists(path):
@@ -76,7 +91,8 @@ def tune_batch(batch, q, qd, qdd, tau, ops, use_cache=True, candidates=None, lan
     def measure(shape, lanes, reps=5, record=True):
         batch.set_launch(*shape)
         batch.set_lanes(lanes)
-        ms = _time(lambda: batch.step(q, qd, qdd, tau, ops, out), reps=reps)
+        with _fp64_kernels(batch) if hasattr(batch, "set_fp64") else contextlib.nullcontext():
+            ms = _time(lambda: batch.step(q, qd, qdd, tau, ops, out), reps=reps)
         if record:
             table.append({"shape": list(shape), "lanes": list(lanes), "ms": ms})
         return ms

@@ -227,6 +227,7 @@ struct sgdyn_batch {
   // the block-floating-point sweep serves the batch when it can hold every model: a launch per
   // model, with each model's tables (its BJoint constants behind them) at offsets_host
   bool bfp = false;
+  bool fp64 = false;  // the caller's choice, whatever `bfp`
   std::vector<BfpTree> trees;
   std::vector<int64_t> offsets_host;
   int4* rest_tiles = nullptr;  // the tiles of the models with one lane per environment
@@ -500,6 +501,15 @@ int sgdyn_batch_set_lanes(sgdyn_batch* b, const int* lanes_per_model) {
   return SGDYN_OK;
 }
 
+int sgdyn_batch_route(sgdyn_batch* b, int fp64, int* fp64_out, int* block_sweep) {
+  if (!b) return set_last_error(SGDYN_ERR_NULL, "null batch");
+  if (fp64 < -1 || fp64 > 1) return set_last_error(SGDYN_ERR_RUNTIME, "fp64 must be -1, 0 or 1");
+  if (fp64 >= 0) b->fp64 = fp64 != 0;
+  if (fp64_out) *fp64_out = b->fp64 ? 1 : 0;
+  if (block_sweep) *block_sweep = b->bfp && !b->fp64 && !fp64_forced() ? 1 : 0;
+  return SGDYN_OK;
+}
+
 int sgdyn_batch_integrate(sgdyn_batch* b, double dt, double* q, double* qd, const double* qdd, void* stream) {
   SG_TRACE("sgdyn_batch_integrate");
   if (!b) return set_last_error(SGDYN_ERR_NULL, "null batch");
@@ -622,7 +632,7 @@ static int batch_step(sgdyn_batch* b, int ops, const double* q, const double* qd
   // op sets beyond these are refused below
   const bool known = ops == (OP_CRBA | OP_RNEA | OP_ABA) || ops == (OP_RNEA | OP_ABA) || ops == OP_ALL ||
                      ops == OP_RNEA || ops == OP_ABA || ops == OP_CRBA;
-  if (b->bfp && known && !fp64_forced()) return batch_step_bfp(b, ops, a.io, integrate, dt, s);
+  if (b->bfp && known && !b->fp64 && !fp64_forced()) return batch_step_bfp(b, ops, a.io, integrate, dt, s);
   // models run with teams: the specialised one-warp-per-role sweep when it is available for
   // every one of them (run-time compilation on, sizes within its limits), each on a side
   // stream of the batch beside the persistent kernel, which takes the remaining tiles

@@ -77,6 +77,25 @@ class HeteroBatch:
             N.check(N.load().sgdyn_batch_set_lanes(self._h, arr))
         self.lanes = tuple(lanes)
 
+    def _route(self, fp64):
+        was, block = ctypes.c_int(), ctypes.c_int()
+        N.check(N.load().sgdyn_batch_route(self._h, fp64, ctypes.byref(was), ctypes.byref(block)))
+        return bool(was.value), bool(block.value)
+
+    @property
+    def block_sweep(self):
+        """Whether steps take the block sweep as the settings stand, not the FP64 kernels that
+        `set_launch` and `set_lanes` shape."""
+        return self._route(-1)[1]
+
+    @property
+    def fp64(self):
+        """Whether this batch was told to run the FP64 kernels (`set_fp64`)."""
+        return self._route(-1)[0]
+
+    def set_fp64(self, on):
+        self._route(1 if on else 0)
+
     # -- padding helpers ------------------------------------------------------------
     def _pad(self, per_model, width, attr):
         out = torch.zeros(self.n, width, dtype=torch.float64, device=self.device)
