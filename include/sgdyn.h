@@ -374,9 +374,9 @@ int sgdyn_rollout_forward(const sgdyn_model* m, int64_t n, int T, double dt, con
 /* Lanes per environment of the ABA-based sweeps: sgdyn_rollout_forward, the reverse sweep
  * of sgdyn_rollout_backward / _noalloc, and forward dynamics requested alone
  * (sgdyn_compute_forward_dynamics, sgdyn_step with only SGDYN_OP_FORWARD_DYNAMICS)
- * (addition): 0 automatic (the default: the
- * block sweeps, see sgdyn_step_split; for models they cannot hold
- * three lanes while one warp per ten environments leaves no FP64 scheduler with two warps),
+ * (addition): 0 automatic (the default: the block sweeps, see sgdyn_step_split, but not for
+ * sgdyn_rollout_backward_noalloc, which has FP64 kernels only; there and for models the sweeps
+ * cannot hold three lanes while one warp per ten environments leaves no FP64 scheduler with two warps),
  * 1, or 3 (one lane per Cartesian axis of every spatial quantity, warp shuffles between
  * them, so each lane issues about half the FP64 instructions of one lane per environment;
  * one-DoF joints and a free-flyer root); -1 only reads the
@@ -406,16 +406,16 @@ int sgdyn_rollout_backward(const sgdyn_model* m, int64_t n, int T, double dt, in
                            const double* qdT_bar, double* q0_bar, double* qd0_bar, double* tau_bar, double* scratch,
                            int64_t scratch_bytes, void* stream);
 
-/* Same reverse pass as sgdyn_rollout_backward for callers that must not allocate device
- * memory while they run (real-time loops that reserve everything at start-up, plug-ins
- * whose host owns the memory budget). No counterpart in the reference. Its scratch is a
- * fixed SGDYN_NOALLOC_SCRATCH_BYTES device array that the library holds on every GPU that
- * loads it, until exit; calls needing more (sgdyn_rollout_scratch_bytes) fail with
+/* The reverse pass of sgdyn_rollout_backward, always by its FP64 kernels, for callers that
+ * must not allocate device memory while they run (real-time loops that reserve everything at
+ * start-up, plug-ins whose host owns the memory budget). No counterpart in the reference. Its
+ * scratch is a fixed SGDYN_NOALLOC_SCRATCH_BYTES device array that the library holds on every
+ * GPU that loads it, until exit; calls needing more (sgdyn_rollout_scratch_bytes) fail with
  * SGDYN_ERR_RUNTIME. It calls no allocator: the model must already be on the device
  * (sgdyn_model_upload). Every call looks the array's address up on the current device; the
- * first lookup on a device may load the library's device code, so make one call on each
- * device (n = 0 does only the lookup) before any stream capture. All calls share the
- * array: calls that overlap on the GPU race. */
+ * first lookup on a device may load the library's device code, so make one call on each device
+ * (n = 0 does only the lookup) before any stream capture. All calls share the array: calls
+ * that overlap on the GPU race. */
 #define SGDYN_NOALLOC_SCRATCH_BYTES (64LL << 20)
 int sgdyn_rollout_backward_noalloc(const sgdyn_model* m, int64_t n, int T, double dt, int checkpoint_every,
                                    const double* q_ckpt, const double* qd_ckpt, const double* tau,

@@ -118,3 +118,27 @@ def test_rollout_and_reverse_pass_in_blocks_of_every_size(name, n):
         want = run()
     for i, (a, b) in enumerate(zip(mine, want)):
         assert rel_per_env(*(t.cpu().numpy().reshape(-1, t.shape[-1]) for t in (a, b))) <= 1e-8, i
+
+
+@pytest.mark.parametrize("name", ["arm9", "quadruped"])
+def test_allocation_free_reverse_pass_agrees_with_automatic_settings(name):
+    """The block sweeps of sgdyn_rollout_backward and the FP64 kernels of its allocation-free form."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = ROBOTS[name]()
+    pm, _ = pair(robot)
+    n, T, K, dt = 21, 7, 3, 1e-3
+    q, qd, _, tau = robot.sample(n, seed=3)
+    q, qd, tau = cuda(q, 0.1 * qd, np.repeat(tau[None], T, axis=0))
+    _, _, qc, qdc = AD.rollout_forward(pm, q, qd, tau, dt, K)
+    bars = cuda(np.ones((n, pm.nq_ext)), np.ones((n, pm.nv)))
+    want = AD.rollout_backward(pm, qc, qdc, tau, dt, K, *bars)
+    got = [torch.empty_like(t) for t in want]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    N.check(N.load().sgdyn_rollout_backward_noalloc(pm._h, n, T, dt, K, *map(p, (qc, qdc, tau, *bars, *got)),
+                                                    ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    for g, w in zip(got, want):
+        g, w = (t.movedim(t.dim() - 2, 0).cpu().numpy() for t in (g, w))
+        assert rel_per_env(g, w) <= 1e-10
