@@ -185,7 +185,9 @@ int sgdyn_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const 
 int sgdyn_step_split(int mode, int* mode_out);
 
 /* Whether the block sweep serves the model as the settings stand (addition): 1 or 0 to *serves. 0:
- * one of its constants is out of range, its tree does not fit, or a setting asks for FP64. */
+ * one of its constants is out of range, its tree does not fit, or a setting asks for FP64. Single
+ * calls go to the FP64 kernels for large batches of deep trees, where these are the faster (chains of
+ * more than 16 joints; rollouts and gradients of floating-base trees beyond some 10000 environments). */
 int sgdyn_model_block_sweep(const sgdyn_model* m, int* serves);
 
 /* Lanes per environment for the single-model fused sweep and single-op entry points

@@ -1,6 +1,7 @@
 // Launches of the block-floating-point sweep: environments per block.
 #include "bfp_launch.h"
 #include "bfp_diff.cuh"
+#include "route.h"
 
 #include <map>
 #include <mutex>
@@ -56,6 +57,67 @@ BlkShape blk_shape(const BfpTree& t, bool adjoint, int64_t n) {
   s.threads = unsigned((E * nv + 31) / 32 * 32);
   s.blocks = unsigned((n + E - 1) / E);
   return s;
+}
+
+// The rules below compare the block sweep with the FP64 kernels by what each takes on GB300 (device
+// time, chains of 7 to 56 revolute joints, trees of 2 to 8 branches with and without a free flyer, 1024
+// to 65536 environments). A block sweep's time grows with n from two blocks per multiprocessor on;
+// its price per environment with the tree's depth: levels are walked one after the other, elimination
+// takes steps cubic in a chain's length (the FP64 forward dynamics are linear in it), and the
+// state's size leaves fewer environments resident. An FP64 kernel takes a time of its own, about
+// proportional to the joints, up to a warp per scheduler and grows with n after that.
+namespace {
+constexpr int64_t kMany = 1 << 20;  // a batch that fills the blocks
+double kilobytes(const BfpTree& t) {
+  return double(bfp::blk_bytes(bfp::blk_layout(t.nj, t.nv, t.nq, t.npairs, false), 0, 1)) / 1024;
+}
+bool one_block(const BfpTree& t) { return blk_shape(t, true, kMany).smem > 113 * 1024; }
+// microseconds per environment of forward dynamics in a large batch: chains of 20, 24, 40 and 56
+// joints 0.020, 0.033, 0.12, 0.35; 35-DoF humanoid 0.029; 9 joints on each of 6 legs 0.069
+double solve_cost(const BfpTree& t, const BfpDepth& d) { return 1e-5 * double(d.elimination) + 4e-4 * t.nv; }
+double few_cost(const BfpTree& t, const BfpDepth& d) {
+  return solve_cost(t, d) * (blk_shape(t, false, kMany).envs <= 4 ? 1.3 : 1.0);
+}
+}  // namespace
+
+// Measured crossings, environments. Forward dynamics alone: chains of 24, 30, 40, 56: 11000, 3900, 2700,
+// 1240 (1474 against 580 us at 4096), humanoid 23000, six legs of 9: 13400; with inverse dynamics
+// 13700, 9500, 6100, 2700, none, 17500. The other sets, and all five: 24 to 28000, 16 to 20000, 10 to
+// 12000, 5400 to 6100, none, none. Mass matrices without forward dynamics: none below 20000 and 1.25
+// times at most.
+bool fp64_faster_step(const BfpTree& t, const BfpDepth& d, int ops, int64_t n) {
+  const double joints = t.nj - 1;
+  if ((ops & OP_CRBA) && !(ops & OP_ABA)) return false;
+  if ((ops & OP_ABA) && !(ops & OP_CRBA)) {
+    const double c = few_cost(t, d);
+    if (ops == OP_ABA) return double(n) * (c - 7.5e-4 * t.nv) > 7 * joints;
+    return double(n) * c > 19 * joints && c > 9.5e-4 * t.nv;
+  }
+  // by latency: levels, times the environments that are not resident
+  const double depth = d.levels * kilobytes(t);
+  return double(n) * depth > 230e3 * joints && depth > 8.3 * t.nv;
+}
+// Crossings, forward and reverse pass: chains of 24, 30, 40, 56: 14200, 10000, 2800 to 4200, 1300 to 2800;
+// 18-DoF quadruped 15500 to 16200 (32768, 10 steps: 5.9 against 4.1 ms), humanoid 11300 to 12100,
+// legs 11400 to 16600; chains up to 16 and the 9-DoF arm none. More than 256 threads of 128 registers
+// leave one block per multiprocessor. Up to ten environments per scheduler the FP64 kernels run
+// three lanes on each.
+bool fp64_faster_rollout(const BfpTree& t, const BfpDepth& d, int64_t n) {
+  const double c = few_cost(t, d) * (blk_shape(t, false, kMany).threads > 256 ? 1.8 : 1.0);
+  const int64_t schedulers = 4 * int64_t(multiprocessors());
+  return double(n) * c > (n <= 10 * schedulers ? 10 : 21) * double(t.nj - 1) && c > 1e-3 * t.nv;
+}
+// Crossings: chains of 40 to 56 joints 8600 to 9300 (16384: 1.9 to 2.5 against 1.1 to 1.5 ms); else none
+// but 1.1 times at 65536 for eight legs of 7.
+bool fp64_faster_rnea_vjp(const BfpTree& t, const BfpDepth& d, int64_t n) {
+  return n > 9000 && d.levels > 20 && one_block(t);
+}
+// Crossings: chains of 20, 24, 30, 40, 56: 14000, 14500, 10000, 3600, 3300 (16384 chains of 40: 6.0 against
+// 1.6 ms), eight legs of 7: 10500; quadruped and humanoid about 20000 (24576: 800 against 651 us; 32768:
+// 2325 against 1654); none for chains up to 11 and the 9-DoF arm (65536: 685 against 926).
+bool fp64_faster_aba_vjp(const BfpTree& t, const BfpDepth& d, int64_t n) {
+  const double c = 2 * solve_cost(t, d) * (one_block(t) ? 1.5 : 1.0);
+  return double(n) * c > 34 * double(t.nj - 1) && c > 1.2e-3 * t.nv;
 }
 
 #define SG_STEP(E)                                                                                             \

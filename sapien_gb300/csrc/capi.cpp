@@ -18,6 +18,7 @@
 #include "jit.h"
 #include "kernels.h"
 #include "model.h"
+#include "route.h"
 
 struct sgdyn_model {
   sgdyn::Model* impl;
@@ -228,10 +229,11 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
   a.tau_out = make_arr(tau_out, n, nv, layout);
   a.qdd_out = make_arr(qdd_out, n, nv, layout);
   auto s = static_cast<cudaStream_t>(stream);
-  // With every setting automatic: the block-floating-point sweep, one launch for any op set and
-  // batch size (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings
-  // (lanes, split, forward-dynamics route) and what that sweep cannot hold.
-  if (block_sweep(Mo) && !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
+  // With every setting automatic: the block-floating-point sweep, one launch for any op set
+  // (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings (lanes, split,
+  // forward-dynamics route), what that sweep cannot hold and large batches of deep trees.
+  if (block_sweep(Mo) && !(ops == OP_ABA && g_rollout_lanes.load() != 0) &&
+      !fp64_faster_step(bfp_tree(Mo), Mo.depth(), ops, n)) {
     const cudaError_t e = launch_bfp_step(dm, bfp_tree(Mo), ops, a, s);
     if (e == cudaSuccess) return SGDYN_OK;
     if (e != cudaErrorNotSupported)
@@ -731,7 +733,7 @@ int sgdyn_compute_inverse_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(qdd_bar, n, nv, layout);
-    if (block_sweep(Mo)) {
+    if (block_sweep(Mo) && !fp64_faster_rnea_vjp(bfp_tree(Mo), Mo.depth(), n)) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::rnea_vjp, dm, bfp_tree(Mo), nullptr, &a,
                                             static_cast<cudaStream_t>(stream));
       if (e != cudaErrorNotSupported) return launch_status(e);
@@ -767,13 +769,7 @@ int sgdyn_compute_forward_dynamics_vjp(const sgdyn_model* m, int64_t n, const do
     a.o1 = make_arr(q_bar, n, nv, layout);
     a.o2 = make_arr(qd_bar, n, nv, layout);
     a.o3 = make_arr(tau_bar, n, nv, layout);
-    // The integer sweep's cost grows with the tree's pairs and with n, the FP64 kernel's is flat up
-    // to a warp per scheduler: with long ancestor chains that one is the faster beyond it
-    // (18-DoF quadruped, 6.5 pairs per column, 16384 environments: 533 us against 556 in FP64,
-    // 24576: 800 against 651; 35-DoF humanoid, 32768: 2325 against 1654; 9-DoF arm, 4.9 pairs,
-    // 131072: 1371 against 1637).
-    const bool long_chains = Mo.btree().npairs > 6 * Mo.nv();
-    if (block_sweep(Mo) && !(long_chains && n > 32 * int64_t(device_schedulers()))) {
+    if (block_sweep(Mo) && !fp64_faster_aba_vjp(bfp_tree(Mo), Mo.depth(), n)) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::aba_vjp, dm, bfp_tree(Mo), nullptr, &a,
                                             static_cast<cudaStream_t>(stream));
       if (e != cudaErrorNotSupported) return launch_status(e);
@@ -906,7 +902,7 @@ int sgdyn_rollout_forward(const sgdyn_model* m, int64_t n, int T, double dt, con
     a.qT = qT; a.qdT = qdT; a.q_ckpt = q_ckpt; a.qd_ckpt = qd_ckpt;
     std::string why;
     const auto st = static_cast<cudaStream_t>(stream);
-    if (block_sweep(Mo) && g_rollout_lanes.load() == 0) {
+    if (block_sweep(Mo) && g_rollout_lanes.load() == 0 && !fp64_faster_rollout(bfp_tree(Mo), Mo.depth(), n)) {
       const cudaError_t e = launch_bfp_diff(BfpDiff::rollout, dm, bfp_tree(Mo), &a, nullptr, st);
       if (e != cudaErrorNotSupported) return launch_status(e);
     }
@@ -1024,7 +1020,8 @@ int sgdyn_rollout_backward(const sgdyn_model* m, int64_t n, int T, double dt, in
     a.q0_bar = q0_bar; a.qd0_bar = qd0_bar; a.tau_bar = tau_bar; a.scratch = scratch;
     const cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nj = Mo.njoints();
-    if (block_sweep(Mo) && g_rollout_lanes.load() == 0 && T > 0) {
+    if (block_sweep(Mo) && g_rollout_lanes.load() == 0 && T > 0 &&
+        !fp64_faster_rollout(bfp_tree(Mo), Mo.depth(), n)) {
       // its records are smaller than the intermediates the scratch is sized for
       const BfpTree tree = bfp_tree(Mo);
       const int64_t seg = bfp_record_doubles(tree) * checkpoint_every * n;

@@ -719,7 +719,9 @@ void Model::rebuild_bfp() {
       ext[a] = J[i].vcol + k;
     }
   }
+  elimination_ = 0;
   for (int a = 0; a < nv; a++) {
+    elimination_ += int64_t(dep[a]) * (dep[a] + 1) / 2;
     rs[a] = int(pr.size());
     std::vector<int> up;
     for (int c = a; c >= 0; c = par[c]) up.push_back(c);

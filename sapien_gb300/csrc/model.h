@@ -64,6 +64,13 @@ struct HostBody {  // a BODY frame (one per URDF link)
   Placement placement;
 };
 
+// Depth of a tree: levels of its columns, and steps of the elimination of M (d (d + 1) / 2 for a
+// column below d others).
+struct BfpDepth {
+  int levels;
+  int64_t elimination;
+};
+
 class Model {
  public:
   // Builds from URDF XML; the root link is welded to the universe (joint 0).
@@ -109,6 +116,7 @@ class Model {
   const std::vector<unsigned char>& bfp_table() const { return bfp_; }
   bool bfp_ok() const { return bfp_ok_; }
   const BTree& btree() const { return btree_; }
+  BfpDepth depth() const { return {btree_.col_levels, elimination_}; }
 
   // Team table for L lanes per environment (layout in step_kernel.cuh: TeamLanes);
   // *critical_path receives the joint-cost length of the trunk + heaviest lane.
@@ -144,6 +152,7 @@ class Model {
   std::vector<unsigned char> bfp_;
   bool bfp_ok_ = false;
   BTree btree_{};
+  int64_t elimination_ = 0;  // see BfpDepth
   std::map<int, void*> dev_;       // device ordinal -> device copy of table_
   std::map<std::pair<int, int>, void*> dev_team_;  // (device, L) -> device team table
   std::map<int, int> team_cp_;                       // L -> critical path

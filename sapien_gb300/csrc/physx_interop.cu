@@ -16,6 +16,7 @@
 #include "../../include/sgdyn.h"
 #include "trace.h"
 #include "model.h"
+#include "route.h"
 #include "step_kernel.cuh"
 
 struct sgdyn_model {
@@ -92,8 +93,8 @@ extern "C" int sgdyn_compute_passive_force_f32(const sgdyn_model* m, int64_t n, 
   const unsigned blocks = unsigned((n + 31) / 32);
   auto s = static_cast<cudaStream_t>(stream);
   // block floating point (bfp_block.cuh): 4096 9-DoF arms 102 -> 29 us; the FP64 kernel below
-  // for models it cannot hold and settings that ask for FP64
-  if (block_sweep(Mo)) {
+  // for models it cannot hold, settings that ask for FP64 and large batches of deep trees
+  if (block_sweep(Mo) && !fp64_faster_step(bfp_tree(Mo), Mo.depth(), OP_RNEA, n)) {
     const cudaError_t e = launch_bfp_passive(dm, bfp_tree(Mo), a, s);
     if (e == cudaSuccess) return SGDYN_OK;
     if (e != cudaErrorNotSupported)
