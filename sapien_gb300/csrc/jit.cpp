@@ -408,6 +408,13 @@ CUfunction get_function(const Model& M, int kind, int ops, std::string* why) {
   return fn;
 }
 
+// Whether get_function has the kernel without compiling or loading it.
+bool function_ready(const Model& M, int kind, int ops) {
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess &&
+         g_by_model.count(std::make_tuple(M.uid(), M.table_version(), kind, ops, dev)) != 0;
+}
+
 CUfunction get_function_slow(const Model& M, int kind, int ops, int dev, std::string* why) {
   Api& A = api();
   const std::string src = generate_source(M, kind, ops);
@@ -578,6 +585,13 @@ bool launch_jit(Model& M, int kind, int ops, const Args& a, cudaStream_t s, std:
     }
     if ((joints >= 0 ? joints : M.njoints()) > g_max_joints) {
       *why = "tree above the run-time compilation size limit";
+      return false;
+    }
+    // loading a module would end the capture with an error
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
+    if (cs != cudaStreamCaptureStatusNone && !function_ready(M, kind, ops)) {
+      *why = "not compiled before the capture";
       return false;
     }
     fn = get_function(M, kind, ops, why);

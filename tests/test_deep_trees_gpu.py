@@ -104,3 +104,31 @@ def test_passive_forces(n, takes_fp64):
     if takes_fp64:
         assert (mine == want).all()
     assert rel_per_env(mine.double().cpu().numpy(), want.double().cpu().numpy()) <= 2.0**-23
+
+
+@pytest.mark.parametrize("what", ["rollout", "product"])
+def test_first_call_under_capture(what):
+    """A call that changes over to kernels compiled at run time, captured before any of them is there."""
+    import torch
+
+    from sapien_gb300 import autodiff as AD
+
+    robot = syn.quadruped(seed=71 if what == "rollout" else 72)
+    pm, _ = pair(robot)
+    n = 24000
+    q, qd, _, tau = cuda(*robot.sample(n, seed=6))
+    pm._prepare(q.device)
+    if what == "rollout":
+        def run():
+            return AD.rollout_forward(pm, q, qd, tau[None], 1e-4)[:2]
+    else:
+        def run():
+            return AD.forward_dynamics_vjp(pm, q, qd, tau, qd)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        captured = run()
+    g.replay()
+    direct = run()
+    torch.cuda.synchronize()
+    for a, b in zip(captured, direct):
+        assert rel_per_env(a.cpu().numpy(), b.cpu().numpy()) <= 1e-9
