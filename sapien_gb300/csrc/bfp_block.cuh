@@ -18,11 +18,11 @@
 //
 // Measured (GB300, device time per call; before: the FP64 sweeps, specialised per model or in
 // teams of lanes, that still serve forced settings and models out of range). All five ops: 7-DoF
-// arm, 16 environments 143 -> 32 us, 1000: 145 -> 33 us; 9-DoF arm, 16384: 156 -> 96 us. CRBA +
-// RNEA + forward dynamics: 9-DoF arm, 131071: 792 -> 544 us; 35-DoF humanoid, 1024: 422 -> 68 us.
-// Forward dynamics alone, 18-DoF quadruped, 3001: 84 -> 41 us. What bounds it at 16384 9-DoF
-// arms: 2381 warp instructions per environment (170 of its thread instructions in FP64, before
-// 4215) issued at 34 % of the schedulers' rate, waiting at barriers and for instruction fetch.
+// arm, 16 environments 143 -> 33 us, 1000: 145 -> 36 us; 9-DoF arm, 16384: 156 -> 98 us. CRBA +
+// RNEA + forward dynamics: 9-DoF arm, 131071: 792 -> 563 us; 35-DoF humanoid, 1024: 422 -> 71 us.
+// Forward dynamics alone, 18-DoF quadruped, 3001: 84 -> 43 us. What bounds it at 16384 9-DoF
+// arms: 2482 warp instructions per environment (170 of its thread instructions in FP64, before
+// 4215) issued at 33 % of the schedulers' rate, waiting at barriers and for instruction fetch.
 #pragma once
 #include "bfp.cuh"
 #include "se3.cuh"
@@ -70,10 +70,11 @@ SG_HD BlkLayout blk_layout(int nj, int nv, int nq, int npairs, bool adjoint = fa
   return L;
 }
 // What a sweep notes of an environment on its way, for the question whether its results have to
-// come from the FP64 algebra (Blk::refused). All but NOTE_REFUSED are the largest binary exponent
+// come from the FP64 algebra (Blk::refused). All after the first two are the largest binary exponent
 // of something, kNoNote where there was nothing.
 enum Note : int {
   NOTE_REFUSED,  // an input, a pivot or an adjoint out of range
+  NOTE_ALIGNED,  // a joint's rotation maps an axis of its frame on one of the world's, or nearly
   NOTE_SCALE,    // products that the bodies' forces are summed from
   NOTE_BIAS,     // generalised bias forces (inverse dynamics)
   NOTE_DRIVE,    // applied generalised forces
@@ -420,7 +421,7 @@ struct Blk {
   __device__ __forceinline__ int& note_at(int s, int note) const { return note_base[(s * kNotes + note) * EI + el]; }
   __device__ __forceinline__ void clear_notes(int s) const {
     if (slot == 0) {
-      for (int k = 0; k < kNotes; k++) note_at(s, k) = k == NOTE_REFUSED ? 0 : kNoNote;
+      for (int k = 0; k < kNotes; k++) note_at(s, k) = k <= NOTE_ALIGNED ? 0 : kNoNote;
     }
   }
   __device__ __forceinline__ void refuse() const {
@@ -439,7 +440,11 @@ struct Blk {
   // FP64 only. lost = kLost: where a row is below 2^-7 of its terms, so that an error of 2^-57 of
   // the terms is at most 2^-50 of the row. Gradients (kLostGrad) are often that much smaller
   // than their terms about the world's origin, where FP64 loses as much: 2^-45 of the row, about
-  // FP64's own error for 9-DoF arms. Results that cancel against applied forces cancel in FP64 too.
+  // FP64's own error for 9-DoF arms. Results that cancel against applied forces cancel in FP64 too,
+  // and so does everything where no rotation is aligned with the world's axes (NOTE_ALIGNED): among
+  // dense rotations FP64's terms are off by 2^-53 of themselves. (6-DoF arms that spin fast about
+  // dense axes have such rows: of 4096, some in most steps of a rollout, 26 -> 27 to 53 us a step
+  // without this.)
   __device__ __forceinline__ bool refused(int lost = kLost) const {
     if constexpr (!A::kFixed) return false;
     const int scale = note_at(set, NOTE_SCALE), least = scale - lost, bias = note_at(set, NOTE_BIAS);
@@ -447,8 +452,10 @@ struct Blk {
     const bool driven = (drive != kNoNote || torque != kNoNote) && (drive == kNoNote || drive >= least) &&
                         (torque == kNoNote || torque >= least);
     const int gscale = note_at(set, NOTE_GSCALE);
-    return note_at(set, NOTE_REFUSED) != 0 || (scale > kTiny && bias != kNoNote && bias < least && !driven) ||
-           (gscale > kTiny && note_at(set, NOTE_GRAD) < gscale - kLostGrad);
+    return note_at(set, NOTE_REFUSED) != 0 ||
+           (note_at(set, NOTE_ALIGNED) != 0 &&
+            ((scale > kTiny && bias != kNoNote && bias < least && !driven) ||
+             (gscale > kTiny && note_at(set, NOTE_GRAD) < gscale - kLostGrad)));
   }
   static constexpr int kTiny = -600;  // below: the terms are 0
 };
@@ -473,6 +480,8 @@ __device__ __forceinline__ typename A::Rot joint_rotation(const DJoint& J, const
 // its row and column below 2^-10), as with joint axes along the frames' axes or on a root joint.
 // (Of a quaternion: where two components are small.)
 constexpr i64 kAligned = kOne - (kOne >> 21);
+// (for NOTE_ALIGNED: the others of its row and column below 2^-7, which is kLost)
+constexpr i64 kNearlyAligned = kOne - (kOne >> 15);
 template <class A, int E, int EI>
 __device__ __forceinline__ void blk_check_configuration(const Blk<A, E, EI>& b) {
   if constexpr (!A::kFixed) return;
@@ -513,14 +522,21 @@ __device__ __forceinline__ void blk_poses(const Blk<A, E, EI>& b) {
 #pragma unroll 1
     for (int k = b.slot; k < n; k += b.slots) {
       const int j = b.order[lo + k / 3], r = k % 3, p = b.parent[j], o = b.iR(j) + 3 * r, im = b.iM(j);
+      i64 v[3];
       if (p == 0) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) b.W(o + c) = b.W(im + 3 * r + c);
+        for (int c = 0; c < 3; c++) v[c] = b.W(im + 3 * r + c);
       } else {
         const int pr = b.iR(p) + 3 * r;
         const i64 r0 = b.W(pr), r1 = b.W(pr + 1), r2 = b.W(pr + 2);
 #pragma unroll
-        for (int c = 0; c < 3; c++) b.W(o + c) = A::row_dot(r0, r1, r2, b.W(im + c), b.W(im + 3 + c), b.W(im + 6 + c));
+        for (int c = 0; c < 3; c++) v[c] = A::row_dot(r0, r1, r2, b.W(im + c), b.W(im + 3 + c), b.W(im + 6 + c));
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) b.W(o + c) = v[c];
+      if constexpr (A::kFixed) {
+        constexpr unsigned least = unsigned(kNearlyAligned >> 32);
+        if (abs_hi(v[0]) >= least || abs_hi(v[1]) >= least || abs_hi(v[2]) >= least) b.note_at(b.set, NOTE_ALIGNED) = 1;
       }
     }
     __syncthreads();
