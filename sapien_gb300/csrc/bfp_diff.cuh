@@ -15,7 +15,7 @@
 //
 // Measured (before: the FP64 kernels, specialised per model): values and gradients of inverse and
 // forward dynamics, 16384 9-DoF arms, 720 -> 605 us; a rollout of 4096 of them over 200 steps with
-// a checkpoint every 20 and its reverse pass, 29.9 -> 19.05 ms (6.2 forward, of the rest two
+// a checkpoint every 20 and its reverse pass, 29.9 -> 19.4 ms (6.3 forward, of the rest two
 // thirds the reverse pass). What bounds them: instruction issue between barriers, the reverse
 // pass besides by its 4096 environments, one block and a bit per multiprocessor.
 #pragma once

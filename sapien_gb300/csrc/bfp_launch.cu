@@ -43,7 +43,7 @@ int multiprocessors() {
 // fewest instructions: 262144 9-DoF arms, CRBA + RNEA + forward dynamics, 1115 us against 1204
 // with 16 and 1556 with 8), as many as leave room for two blocks per multiprocessor (110 KB
 // each), so that one computes while the other waits at a barrier; fewer while the batch has
-// less than two blocks per multiprocessor (3001 quadrupeds: 77 us with 8, 83 with 16). 0: not
+// less than two blocks per multiprocessor. 0: not
 // even four environments fit a block.
 BlkShape blk_shape(const BfpTree& t, bool adjoint, int64_t n) {
   const bfp::BlkLayout L = bfp::blk_layout(t.nj, t.nv, t.nq, t.npairs, adjoint);
