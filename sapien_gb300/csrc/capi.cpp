@@ -232,8 +232,8 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
   // With every setting automatic: the block-floating-point sweep, one launch for any op set
   // (bfp_block.cuh; figures there). The FP64 sweeps below serve forced settings (lanes, split,
   // forward-dynamics route), what that sweep cannot hold and large batches of deep trees.
-  if (block_sweep(Mo) && !(ops == OP_ABA && g_rollout_lanes.load() != 0) &&
-      !fp64_faster_step(bfp_tree(Mo), Mo.depth(), ops, n)) {
+  const bool block = block_sweep(Mo), deep = block && fp64_faster_step(bfp_tree(Mo), Mo.depth(), ops, n);
+  if (block && !deep && !(ops == OP_ABA && g_rollout_lanes.load() != 0)) {
     const cudaError_t e = launch_bfp_step(dm, bfp_tree(Mo), ops, a, s);
     if (e == cudaSuccess) return SGDYN_OK;
     if (e != cudaErrorNotSupported)
@@ -260,7 +260,9 @@ int run_step(const sgdyn_model* m, int64_t n, int ops, const double* q, const do
     cudaError_t e = launch_aba3(dm, Mo.njoints(), a, s);
     if (e != cudaSuccess) return fail(SGDYN_ERR_CUDA, std::string("kernel launch failed: ") + cudaGetErrorString(e));
     return SGDYN_OK;
-  } else if (ops == OP_ALL && use_split(n)) {
+  } else if (ops == OP_ALL && !(deep && bfp_step_fits(bfp_tree(Mo))) && use_split(n)) {
+    // (in one launch for deep trees: chains of 24, 30, 40 and 56, 24576 environments, 1039, 1416, 2203
+    // and 3776 us against 1306, 1757, 2662 and 4386 in two)
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) cs = cudaStreamCaptureStatusActive;
     cudaStream_t s2 = cs == cudaStreamCaptureStatusNone ? side_stream() : nullptr;

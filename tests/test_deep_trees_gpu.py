@@ -44,7 +44,7 @@ FK, RNEA, ABA, CRBA = N.OP_FK, N.OP_INVERSE_DYNAMICS, N.OP_FORWARD_DYNAMICS, N.O
     ("chain40", 1000, ABA, False), ("chain40", 4000, ABA, True), ("chain40", 4000, ABA | RNEA, False),
     ("chain40", 8000, ABA | RNEA, True), ("chain40", 8000, FK, False), ("chain40", 13000, FK, True),
     ("chain40", 13000, RNEA, True), ("chain40", 13000, CRBA | RNEA | ABA, True), ("chain40", 13000, CRBA, False),
-    ("chain16", 40000, ABA, False), ("humanoid", 12000, ABA, False), ("quadruped", 40000, ABA, False)])
+    ("chain40", 13000, N.OP_ALL, True), ("chain16", 40000, ABA, False), ("humanoid", 12000, ABA, False), ("quadruped", 40000, ABA, False)])
 def test_steps(name, n, ops, takes_fp64):
     robot = robot_of(name)
     pm, _ = pair(robot)
